@@ -133,6 +133,25 @@ template <> struct Shape<K_COS> { // w = 4 cos(pi q) + cos(2 pi q) + 3
     }
 };
 
+// One-instruction forms of 1 / sqrt and the product that follows it: for
+// normal arguments the same bits as rsqrtf and *, without the scaling that
+// rsqrtf carries for subnormal ones (three more instructions per pair). A
+// subnormal argument counts as 0: rsqrt_ftz(0) is +inf and mul_ftz(0, +inf)
+// NaN, which a saturating operation turns into 0.
+__device__ __forceinline__ float rsqrt_ftz(float a)
+{
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+    return r;
+}
+
+__device__ __forceinline__ float mul_ftz(float a, float b)
+{
+    float r;
+    asm("mul.rn.ftz.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
 // W and the gradient factor g (grad W = g * x_ij) for a neighbour pair with
 // squared distance 0 <= l2 <= r^2 (the traversal guarantees the range).
 // len = l2 * rsqrt(l2) replaces the reference's norm3df; the self pair
@@ -140,8 +159,8 @@ template <> struct Shape<K_COS> { // w = 4 cos(pi q) + cos(2 pi q) + 3
 template <int KIND>
 __device__ __forceinline__ float pair_w(const KernelConst& k, float l2)
 {
-    const float len = l2 > 0.f ? l2 * rsqrtf(l2) : 0.f;
-    return k.w_scale * Shape<KIND>::w(__saturatef(len * k.h_inv));
+    // l2 = 0: NaN saturates to q = 0
+    return k.w_scale * Shape<KIND>::w(__saturatef(mul_ftz(l2, rsqrt_ftz(l2)) * k.h_inv));
 }
 
 template <int KIND, class = void> struct HasDwOverQ {
@@ -152,23 +171,27 @@ struct HasDwOverQ<KIND, decltype(void(Shape<KIND>::kDwOverQ))> {
     static constexpr bool value = Shape<KIND>::kDwOverQ;
 };
 
+// 1 / |x| of a pair, finite at l2 = 0, where the length l2 * inv_length(l2)
+// is then 0 and every kernel's dw(0) as well, so that g = dw(0) inv is the
+// zero that the reference's non-finite guard gives (kernels.cuh:51-64)
+__device__ __forceinline__ float inv_length(float l2) { return rsqrt_ftz(fmaxf(l2, 1e-30f)); }
+
 // the gradient factor g with grad W(x) = g x. For the Wendland kernels dw(q)
 // carries a factor q, so g = dw_scale / h_bar * dw(q) / q needs no division
 // by |x|; at x = 0 it is finite and multiplies a zero vector. Otherwise the
-// reference's form dw_scale * dw(q) / |x| with its non-finite guard
-// (kernels.cuh:51-64).
+// reference's form dw_scale * dw(q) / |x|.
 template <int KIND>
 __device__ __forceinline__ float pair_g(const KernelConst& k, float l2)
 {
-    const float inv = rsqrtf(l2);
-    if constexpr (HasDwOverQ<KIND>::value) {
-        // coincident points (l2 = 0) get the finite g at q = 0
-        const float len = l2 > 0.f ? l2 * inv : 0.f;
-        return (k.dw_scale * k.h_inv) * Shape<KIND>::dw_over_q(len * k.h_inv);
+    if constexpr (KIND == K_C2) { // dw_over_q; l2 = 0: NaN saturates to 0
+        const float t = __saturatef(fmaf(-mul_ftz(l2, rsqrt_ftz(l2)), k.h_inv, 1.f));
+        return (k.dw_scale * k.h_inv) * (t * t * t * -20.f);
     } else {
-        const float len = l2 * inv;
-        const float g = k.dw_scale * Shape<KIND>::dw(len * k.h_inv) * inv;
-        return (l2 > 0.f && isfinite(g)) ? g : 0.f;
+        const float inv = inv_length(l2);
+        if constexpr (HasDwOverQ<KIND>::value)
+            return (k.dw_scale * k.h_inv) * Shape<KIND>::dw_over_q(l2 * inv * k.h_inv);
+        else
+            return k.dw_scale * Shape<KIND>::dw(l2 * inv * k.h_inv) * inv;
     }
 }
 
@@ -176,12 +199,10 @@ template <int KIND>
 __device__ __forceinline__ void pair_wg(
     const KernelConst& k, float l2, float& w, float& g)
 {
-    const float inv = rsqrtf(l2);
-    const float len = l2 > 0.f ? l2 * inv : 0.f;
-    const float q = len * k.h_inv;
+    const float inv = inv_length(l2);
+    const float q = l2 * inv * k.h_inv;
     w = k.w_scale * Shape<KIND>::w(__saturatef(q));
-    const float gg = k.dw_scale * Shape<KIND>::dw(q) * inv;
-    g = (l2 > 0.f && isfinite(gg)) ? gg : 0.f;
+    g = k.dw_scale * Shape<KIND>::dw(q) * inv;
 }
 
 // ---- uniform grid view ----------------------------------------------------
@@ -393,25 +414,105 @@ __device__ __forceinline__ void for_each_row(const GridView& g, int3 c, float xi
     }
 }
 
+__device__ __forceinline__ float fast_sqrt(float a)
+{
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+    return r;
+}
+
+// The rows of for_each_row in XYZ order, with the trim in few instructions:
+// run(s, e) gets the sorted range of a row's particles. The traversal is bound
+// by instruction issue (about 21 rows and 80 candidates for 29 neighbours), so
+// the floors of the chord's ends come from one rounded-down addition of
+// 1.5 * 2^23 each, whose low mantissa bits then hold the integer: no
+// float-to-integer conversion, no test for an empty row. f.x is held to
+// [-R, R + 1] for that, which keeps every index inside the prefix (only points
+// clamped into the grid lie outside [0, 1], and a point beyond that range has
+// no candidate within r). The prefix of a slab's rows is loaded before their
+// candidates, so that the loads overlap.
+template <int R, class Run>
+__device__ __forceinline__ void for_each_row_xyz(const GridView& g, int3 c, float xi, float yi,
+    float zi, Run&& run)
+{
+    constexpr float EPS = 1e-3f;
+    constexpr float BIG = 12582912.f; // 1.5 * 2^23
+    const RowFrame fr = row_frame(g, c, xi, yi, zi);
+    const float fx = fminf(fmaxf(fr.fx, -(float)R), (float)(R + 1));
+    const float xl = fx - EPS, xh = fx + EPS;
+    float gy2[2 * R + 1];
+#pragma unroll
+    for (int dy = -R; dy <= R; ++dy) {
+        const float gy = dy > 0 ? fmaxf((float)dy - fr.fy, 0.f)
+                                : (dy < 0 ? fmaxf(fr.fy - (float)(dy + 1), 0.f) : 0.f);
+        gy2[dy + R] = gy * gy;
+    }
+    // the key of the point's own cell, less the bits of BIG
+    uint32_t kz = uint32_t((c.z - R) * g.nxny + (c.y - R) * g.nx + c.x) - __float_as_uint(BIG);
+#pragma unroll 1
+    for (int dz = -R; dz <= R; ++dz, kz += uint32_t(g.nxny)) {
+        const float t0 = fr.rr - slab_gap2(fr, dz);
+        if (t0 < 0.f)
+            continue;
+        uint32_t s[2 * R + 1], e[2 * R + 1];
+        uint32_t ky = kz;
+#pragma unroll
+        for (int u = 0; u <= 2 * R; ++u, ky += uint32_t(g.nx)) {
+            const float t = t0 - gy2[u];
+            const float w = fast_sqrt(fmaxf(t, 0.f)); // half chord, cells
+            const uint32_t a = __float_as_uint(__fadd_rd(fmaxf(xl - w, -(float)R), BIG));
+            const uint32_t b = __float_as_uint(__fadd_rd(fminf(xh + w, (float)R), BIG));
+            s[u] = e[u] = 0;
+            if (t >= 0.f) {
+                s[u] = __ldg(g.prefix + (ky + a));
+                e[u] = __ldg(g.prefix + (ky + b + 1u));
+            }
+        }
+#pragma unroll
+        for (int u = 0; u <= 2 * R; ++u)
+            run(s[u], e[u]);
+    }
+}
+
 // Fixed-radius neighbour traversal: f(j, pts[j], dx, dy, dz, l2) for every
 // candidate with l2 <= r^2 (self included, as the reference's accumulation
 // does), in the reference's row order. `pts` are packed (x, y, z, mass) in
 // grid order.
-template <int R, class F>
+// XYZ: the grid is in XYZ order (the caller knows; false serves both orders).
+// On the 4M dam break from rest the density pass over these loops takes 502 us
+// against 747 us over for_each_row with the compiler's own unrolling of the
+// candidate loop (by four, for rows of three to five candidates); one
+// candidate a round 508 us, two with a clamped second index 566 us, five
+// rows' candidates as 64-bit pointer loops 599 us, one load ahead 704 us.
+template <int R, bool XYZ = false, class F>
 __device__ __forceinline__ void for_each_neighbour(const GridView& g, int3 c,
     float xi, float yi, float zi, const float4* __restrict__ pts, F&& f)
 {
-    for_each_row<R>(g, c, xi, yi, zi, [&](uint32_t k0, int ncell) {
-        const uint32_t s = __ldg(g.prefix + k0);
-        const uint32_t e = __ldg(g.prefix + k0 + ncell);
-        for (uint32_t j = s; j < e; ++j) {
-            const float4 q = __ldg(pts + j);
-            const float dx = xi - q.x, dy_ = yi - q.y, dz_ = zi - q.z;
-            const float l2 = fmaf(dx, dx, fmaf(dy_, dy_, dz_ * dz_));
-            if (l2 <= g.r2)
-                f(j, q, dx, dy_, dz_, l2);
-        }
-    });
+    auto test = [&](uint32_t j, const float4& q) {
+        const float dx = xi - q.x, dy_ = yi - q.y, dz_ = zi - q.z;
+        const float l2 = fmaf(dx, dx, fmaf(dy_, dy_, dz_ * dz_));
+        if (l2 <= g.r2)
+            f(j, q, dx, dy_, dz_, l2);
+    };
+    if constexpr (XYZ) {
+        for_each_row_xyz<R>(g, c, xi, yi, zi, [&](uint32_t j, uint32_t e) {
+#pragma unroll 1
+            for (; j + 1 < e; j += 2) { // two loads in flight
+                const float4 q0 = __ldg(pts + j), q1 = __ldg(pts + j + 1);
+                test(j, q0);
+                test(j + 1, q1);
+            }
+            if (j < e)
+                test(j, __ldg(pts + j));
+        });
+    } else {
+        for_each_row<R>(g, c, xi, yi, zi, [&](uint32_t k0, int ncell) {
+            const uint32_t e = __ldg(g.prefix + k0 + ncell);
+#pragma unroll 1
+            for (uint32_t j = __ldg(g.prefix + k0); j < e; ++j)
+                test(j, __ldg(pts + j));
+        });
+    }
 }
 
 // ---- counter-based random numbers ------------------------------------------

@@ -731,7 +731,7 @@ void kernel_eval(int kind, float h_bar, const float* dx, const float* dy, const 
 
 // the reference grid test's quantities (uniformgrid.cu:185-207) and the
 // density sum (solver.cuh:31-33), evaluated per grid slot over packed points
-template <int KIND, int R>
+template <int KIND, int R, bool XYZ>
 __global__ void __launch_bounds__(NBR_THREADS) k_neighbour_stats(uint32_t n, GridView g,
     KernelConst kc, const float4* __restrict__ pts, const uint32_t* __restrict__ owner,
     uint32_t* __restrict__ count, float* __restrict__ len2, float* __restrict__ rho,
@@ -750,7 +750,7 @@ __global__ void __launch_bounds__(NBR_THREADS) k_neighbour_stats(uint32_t n, Gri
     }
     uint32_t cnt = 0;
     float l2sum = 0.f, dens = 0.f;
-    for_each_neighbour<R>(g, c, me.x, me.y, me.z, pts,
+    for_each_neighbour<R, XYZ>(g, c, me.x, me.y, me.z, pts,
         [&](uint32_t j, const float4& q, float, float, float, float l2) {
             cnt += (j == s) ? 0u : 1u;
             l2sum += l2;
@@ -789,10 +789,11 @@ static void launch_stats(int range, unsigned b, cudaStream_t s, uint32_t n, Grid
     KernelConst kc, const float4* pts, const uint32_t* owner, uint32_t* count, float* len2,
     float* rho, uint32_t* status)
 {
-    if (range == 2)
-        k_neighbour_stats<KIND, 2><<<b, NBR_THREADS, 0, s>>>(n, g, kc, pts, owner, count, len2, rho, status);
-    else
-        k_neighbour_stats<KIND, 1><<<b, NBR_THREADS, 0, s>>>(n, g, kc, pts, owner, count, len2, rho, status);
+    const bool xyz = g.order == REYN_ORDER_XYZ;
+    auto kern = range == 2
+        ? (xyz ? k_neighbour_stats<KIND, 2, true> : k_neighbour_stats<KIND, 2, false>)
+        : (xyz ? k_neighbour_stats<KIND, 1, true> : k_neighbour_stats<KIND, 1, false>);
+    kern<<<b, NBR_THREADS, 0, s>>>(n, g, kc, pts, owner, count, len2, rho, status);
 }
 
 void neighbour_stats(const Grid& g, const float* x, const float* y, const float* z,
@@ -867,7 +868,7 @@ __global__ void __launch_bounds__(NBR_THREADS) k_boundary_mass(uint32_t n, GridV
     const float4 me = pts[i];
     int3 c = clamp_cell(g, cell_of(g, me.x, me.y, me.z), R);
     float sum = 0.f;
-    for_each_neighbour<R>(g, c, me.x, me.y, me.z, pts,
+    for_each_neighbour<R, true>(g, c, me.x, me.y, me.z, pts,
         [&](uint32_t, const float4& q, float, float, float, float l2) {
             sum += q.w * pair_w<K_B3>(kc, l2);
         });

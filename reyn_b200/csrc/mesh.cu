@@ -857,7 +857,7 @@ namespace {
             c = clamp_cell(g, c, R);
         }
         float sum = 0.f;
-        for_each_neighbour<R>(g, c, me.x, me.y, me.z, pts,
+        for_each_neighbour<R, true>(g, c, me.x, me.y, me.z, pts,
             [&](uint32_t, const float4&, float, float, float, float l2) {
                 sum += pair_w<K_B3>(kc, l2);
             });
@@ -878,7 +878,7 @@ namespace {
         const int3 c = clamp_cell(g, cell_of(g, me.x, me.y, me.z), R);
         const float ti = inv_rho0_sq * nd[s];
         float ax = 0.f, ay = 0.f, az = 0.f;
-        for_each_neighbour<R>(g, c, me.x, me.y, me.z, pts,
+        for_each_neighbour<R, true>(g, c, me.x, me.y, me.z, pts,
             [&](uint32_t j, const float4&, float dx, float dy, float dz, float l2) {
                 const float w = (ti + inv_rho0_sq * __ldg(nd + j)) * pair_g<K_B3>(kc, l2);
                 ax = fmaf(w, dx, ax);

@@ -428,7 +428,7 @@ template <int KIND>
 __device__ __forceinline__ float rec_g(const KernelConst& k, float l2)
 {
     if constexpr (KIND == K_C2) {
-        const float t = fmaxf(0.f, fmaf(-k.h_inv, l2 * rsqrtf(l2), 1.f));
+        const float t = __saturatef(fmaf(-k.h_inv, mul_ftz(l2, rsqrt_ftz(l2)), 1.f));
         return t * t * t;
     } else {
         return pair_g<KIND>(k, l2);
@@ -539,94 +539,107 @@ __device__ __forceinline__ void for_each_boundary(const Bdy& b, float x, float y
         return;
     if (!__ldg(b.near + (c.z * b.g.nxny + c.y * b.g.nx + c.x)))
         return;
-    for_each_neighbour<2>(b.g, c, x, y, z, b.pm, f);
+    for_each_neighbour<2, true>(b.g, c, x, y, z, b.pm, f);
 }
 
-// The density pass's boundary sums (rb = sum_b m_b W_ib and
-// g = sum_b m_b grad W_ib) for every lane of the warp whose cell has samples
-// within reach, computed by the whole warp: for each such lane in turn, lanes
-// 0-24 take one row each of that point's 5x5 rows of boundary cells (the
-// rows and trim of for_each_boundary) and the warp adds the rows up. A lane
-// walking its 25 rows alone holds its warp for all of them; in the batched
-// workloads three warps in four hold a lane near a wall (scene boxes are a
-// few dozen particles wide), so the batched density pass uses this; in one
-// large scene few warps do, and the lanes walk alone there. Every lane of the
-// warp must call this (no lane may have returned); `need_point` says whether
-// the lane's own point is a fluid particle. The sums run over the samples
-// for_each_boundary visits, added in another order. Batched scenes: each
-// point uses its own scene's boundary grid.
+// The density pass's boundary sums of a warp's particles: g = sum_b m_b grad
+// W_ib in x, y, z and sum_b m_b W_ib in w. Where many lanes of the warp have
+// samples within reach (a wall along the warp's run of cells) each walks its
+// own boundary cells; where few do (a wall at the end of the run: one warp in
+// eight on the 4M dam break, three in four in a batch of small scenes) the
+// warp forms each such lane's sums together, one of the 25 rows of cells a
+// lane, instead of waiting for one lane's 25 rows. A row costs a lane alone
+// about as much as a whole point costs the warp together times COOP_LANES /
+// 25. Every lane of the warp calls this; `valid`: the lane has a particle.
+// `b`: the view of the lane's own scene (batched scenes), b0 of all.
+constexpr int COOP_LANES = 6;
+
 template <int KIND, bool BATCH>
-__device__ __forceinline__ float4 boundary_sums_warp(const Bdy& b0, const KernelConst& kc,
-    bool need_point, uint32_t scene, float x, float y, float z)
+__device__ __forceinline__ float4 boundary_sums(const Bdy& b0, const KernelConst& kc, bool valid,
+    uint32_t scene, const float4& me)
 {
     const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    bool need = false;
-    if (need_point && b0.n) {
+    auto of_scene = [&](uint32_t s) {
         Bdy b = b0;
         if constexpr (BATCH) {
-            if (b.g.sid) {
-                b.g = at_scene(b.g, scene);
-                b.near += b.g.key_base;
-            }
-        }
-        const int3 c = cell_of(b.g, x, y, z);
-        need = cell_inside(b.g, c, 2)
-            && __ldg(b.near + (c.z * b.g.nxny + c.y * b.g.nx + c.x)) != 0;
-    }
-    unsigned m = __ballot_sync(FULL, need);
-    float4 mine = make_float4(0.f, 0.f, 0.f, 0.f);
-    while (m) {
-        const int src = __ffs(m) - 1;
-        m &= m - 1;
-        const float px = __shfl_sync(FULL, x, src), py = __shfl_sync(FULL, y, src),
-                    pz = __shfl_sync(FULL, z, src);
-        Bdy b = b0;
-        if constexpr (BATCH) {
-            const uint32_t s = __shfl_sync(FULL, scene, src);
             if (b.g.sid) {
                 b.g = at_scene(b.g, s);
                 b.near += b.g.key_base;
             }
         }
-        float rb = 0.f, gx = 0.f, gy = 0.f, gz = 0.f;
+        return b;
+    };
+    float4 sums = make_float4(0.f, 0.f, 0.f, 0.f);
+    int3 c = make_int3(0, 0, 0);
+    bool need = false;
+    if (valid && b0.n) {
+        const Bdy b = of_scene(scene);
+        c = cell_of(b.g, me.x, me.y, me.z);
+        need = cell_inside(b.g, c, 2)
+            && __ldg(b.near + (c.z * b.g.nxny + c.y * b.g.nx + c.x)) != 0;
+    }
+    unsigned m = __ballot_sync(FULL, need);
+    if (m == 0)
+        return sums;
+    auto add = [&](float4& v, const float4& q, float dx, float dy, float dz, float l2) {
+        float w, g;
+        pair_wg<KIND>(kc, l2, w, g);
+        v.w += q.w * w;
+        const float mg = q.w * g;
+        v.x += mg * dx;
+        v.y += mg * dy;
+        v.z += mg * dz;
+    };
+    if (__popc(m) > COOP_LANES) {
+        if (need) {
+            const Bdy b = of_scene(scene);
+            for_each_neighbour<2, true>(b.g, c, me.x, me.y, me.z, b.pm,
+                [&](uint32_t, const float4& q, float dx, float dy, float dz, float l2) {
+                    add(sums, q, dx, dy, dz, l2);
+                });
+        }
+        return sums;
+    }
+    const int lane = threadIdx.x & 31;
+    const int dz = lane / 5 - 2, dy = lane % 5 - 2;
+    while (m) {
+        const int src = __ffs(m) - 1;
+        m &= m - 1;
+        const float px = __shfl_sync(FULL, me.x, src), py = __shfl_sync(FULL, me.y, src),
+                    pz = __shfl_sync(FULL, me.z, src);
+        const int3 pc = make_int3(__shfl_sync(FULL, c.x, src), __shfl_sync(FULL, c.y, src),
+            __shfl_sync(FULL, c.z, src));
+        const Bdy b = of_scene(BATCH ? __shfl_sync(FULL, scene, src) : 0u);
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (lane < 25) {
-            const int3 c = cell_of(b.g, px, py, pz);
-            const RowFrame fr = row_frame(b.g, c, px, py, pz);
-            const int dz = lane / 5 - 2, dy = lane % 5 - 2;
+            const RowFrame fr = row_frame(b.g, pc, px, py, pz);
             const float gz2 = slab_gap2(fr, dz);
             int x0, x1;
             if (gz2 <= fr.rr && row_span<2>(fr, gz2, dy, x0, x1)) {
                 const uint32_t k0 =
-                    uint32_t((c.z + dz) * b.g.nxny + (c.y + dy) * b.g.nx + c.x + x0);
+                    uint32_t((pc.z + dz) * b.g.nxny + (pc.y + dy) * b.g.nx + pc.x + x0);
                 const uint32_t e = __ldg(b.g.prefix + k0 + uint32_t(x1 - x0 + 1));
+#pragma unroll 1
                 for (uint32_t j = __ldg(b.g.prefix + k0); j < e; ++j) {
                     const float4 q = __ldg(b.pm + j);
-                    const float dx = px - q.x, dyy = py - q.y, dzz = pz - q.z;
-                    const float l2 = fmaf(dx, dx, fmaf(dyy, dyy, dzz * dzz));
-                    if (l2 <= b.g.r2) {
-                        float w, g;
-                        pair_wg<KIND>(kc, l2, w, g);
-                        rb += q.w * w;
-                        const float mg = q.w * g;
-                        gx += mg * dx;
-                        gy += mg * dyy;
-                        gz += mg * dzz;
-                    }
+                    const float dx = px - q.x, ey = py - q.y, ez = pz - q.z;
+                    const float l2 = fmaf(dx, dx, fmaf(ey, ey, ez * ez));
+                    if (l2 <= b.g.r2)
+                        add(v, q, dx, ey, ez, l2);
                 }
             }
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
-            rb += __shfl_xor_sync(FULL, rb, o);
-            gx += __shfl_xor_sync(FULL, gx, o);
-            gy += __shfl_xor_sync(FULL, gy, o);
-            gz += __shfl_xor_sync(FULL, gz, o);
+            v.x += __shfl_xor_sync(FULL, v.x, o);
+            v.y += __shfl_xor_sync(FULL, v.y, o);
+            v.z += __shfl_xor_sync(FULL, v.z, o);
+            v.w += __shfl_xor_sync(FULL, v.w, o);
         }
         if (lane == src)
-            mine = make_float4(gx, gy, gz, rb);
+            sums = v;
     }
-    return mine;
+    return sums;
 }
 
 // jacobi_update (IISPH.cu:108-117). The reference compares the float a_ii
@@ -984,73 +997,51 @@ unsigned persistent_grid(Kern kern, unsigned bs, unsigned tiles)
 // neighbour list, written entry by entry (a block's rows form one 32 KB
 // region, so the L2 merges the scattered 4-byte stores into full lines).
 // MIXED: the particle's FP16 velocity/density record is written for later
-// passes; MIXED_POS16: its 16-byte record for the non-pressure pass. The
-// one-scene MIXED_POS16 form is held to 40 registers (12 blocks of 128 per
-// SM, 16 bytes spilled) like the other modes' forms: on the 4M dam break
-// 753 us per launch against 771 us at the compiler's 47 registers.
-template <int KIND, int R, int MIX = 0, bool BATCH = false, int MB = NBR_THREADS>
-__global__ void __launch_bounds__(MB, ((MIX == MIX_POS16 && !BATCH) ? 65536 / 40 / MB : 0))
+// passes; MIXED_POS16: its 16-byte record for the non-pressure pass.
+// Bound by instruction issue (the cell traversal). One scene: held to 40
+// registers (12 blocks of 128 per SM); 48 registers run slower (514 against
+// 502 us on the 4M dam break in MIXED_POS16), 32 as well (527).
+template <int KIND, int R, bool XYZ, int MIX = 0, bool BATCH = false, int MB = NBR_THREADS>
+__global__ void __launch_bounds__(MB, (BATCH ? 0 : 65536 / 40 / MB))
 k_density(uint32_t n, Fluid f, Bdy b,
     float* __restrict__ rho, float4* __restrict__ vel, float4* __restrict__ bterm,
     uint4* __restrict__ rec_out, uint2* __restrict__ velh_out)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    // batched scenes: every lane stays until the boundary sums, which its warp
-    // forms together
-    if constexpr (!BATCH) {
-        if (i >= n)
-            return;
-    }
-    const bool valid = i < n;
+    const bool valid = i < n; // the boundary sums need the whole warp
+    const float4 me = valid ? f.pm[i] : make_float4(0.f, 0.f, 0.f, 0.f);
     uint32_t scene = 0;
     if constexpr (BATCH) {
         if (valid)
             scene = enter_scene(f, i);
     }
-    const float4 me = valid ? f.pm[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    int3 c = make_int3(0, 0, 0);
+    // before the traversal, while little else is live; read back at the end
+    const float4 bs = boundary_sums<KIND, BATCH>(b, f.kc, valid, scene, me);
+    if (!valid)
+        return;
+    bterm[i] = bs;
+    const int3 c = fluid_cell<R>(f, me);
     uint32_t cnt = 0;
     float rf = 0.f;
-    if (valid) {
-        c = fluid_cell<R>(f, me);
-        uint32_t* __restrict__ row = f.nbr + list_slot(i, 0);
-        [[maybe_unused]] Kahan rk; // mixed modes: compensated density sum
-        for_each_neighbour<R>(f.g, c, me.x, me.y, me.z, f.pm,
-            [&](uint32_t j, const float4& q, float, float, float, float l2) {
-                if constexpr (MIX)
-                    rk.add(q.w * pair_w<KIND>(f.kc, l2));
-                else
-                    rf += q.w * pair_w<KIND>(f.kc, l2);
-                if (j != i) {
-                    if (cnt < KMAX)
-                        row[size_t(cnt) * 128] = j;
-                    ++cnt;
-                }
-            });
-        if constexpr (MIX)
-            rf = rk.sum;
-    }
-    float4 bs = make_float4(0.f, 0.f, 0.f, 0.f);
-    if constexpr (BATCH) {
-        bs = boundary_sums_warp<KIND, BATCH>(b, f.kc, valid, scene, me.x, me.y, me.z);
-        if (!valid)
-            return;
-    } else {
-        for_each_boundary(b, me.x, me.y, me.z,
-            [&](uint32_t, const float4& q, float dx, float dy, float dz, float l2) {
-                float w, g;
-                pair_wg<KIND>(f.kc, l2, w, g);
-                bs.w += q.w * w;
-                const float mg = q.w * g;
-                bs.x += mg * dx;
-                bs.y += mg * dy;
-                bs.z += mg * dz;
-            });
-    }
-    const float r = rf + bs.w;
+    uint32_t* __restrict__ row = f.nbr + list_slot(i, 0);
+    [[maybe_unused]] Kahan rk; // mixed modes: compensated density sum
+    for_each_neighbour<R, XYZ>(f.g, c, me.x, me.y, me.z, f.pm,
+        [&](uint32_t j, const float4& q, float, float, float, float l2) {
+            if constexpr (MIX)
+                rk.add(q.w * pair_w<KIND>(f.kc, l2));
+            else
+                rf += q.w * pair_w<KIND>(f.kc, l2);
+            if (j != i) {
+                if (cnt < KMAX)
+                    row[size_t(cnt) * 128] = j;
+                ++cnt;
+            }
+        });
+    if constexpr (MIX)
+        rf = rk.sum;
+    const float r = rf + reinterpret_cast<const volatile float*>(bterm + i)[3];
     rho[i] = r;
     vel[i].w = r;
-    bterm[i] = bs;
     f.ncount[i] = cnt;
     if constexpr (MIX == MIX_POS16) {
         const float4 v = vel[i];
@@ -1900,9 +1891,14 @@ void solver_step_t(reyn_solver& sv, reyn_particles& st, const Grid& grid,
         constexpr int R = decltype(RC)::value;
         constexpr int MIX = decltype(MC)::value;
         constexpr bool B = decltype(BC)::value;
-        REYN_KERNEL("k_density", s,
-            k_density<K, R, MIX, B, MB><<<nb, bs, 0, s>>>(n, f, b, sv.rho.get(), st.vel.get(),
-            sv.bterm.get(), REC0, VH));
+        if (f.g.order == REYN_ORDER_XYZ)
+            REYN_KERNEL("k_density", s,
+                k_density<K, R, true, MIX, B, MB><<<nb, bs, 0, s>>>(n, f, b, sv.rho.get(),
+                st.vel.get(), sv.bterm.get(), REC0, VH));
+        else
+            REYN_KERNEL("k_density", s,
+                k_density<K, R, false, MIX, B, MB><<<nb, bs, 0, s>>>(n, f, b, sv.rho.get(),
+                st.vel.get(), sv.bterm.get(), REC0, VH));
         if (sv.scheme == REYN_SESPH) {
             REYN_KERNEL("k_sesph", s,
                 k_sesph<K, R, B, MB><<<nb, bs, 0, s>>>(n, f, st.vel.get(), sv.bterm.get(),

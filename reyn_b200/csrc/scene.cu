@@ -142,7 +142,7 @@ __global__ void k_cull_mark(uint32_t n, const float* __restrict__ x, const float
     uint32_t hit = 0;
     const int3 c = cell_of(bg, px, py, pz);
     if (cell_inside(bg, c, 2) && near[c.z * bg.nxny + c.y * bg.nx + c.x]) {
-        for_each_neighbour<2>(bg, c, px, py, pz, bpm,
+        for_each_neighbour<2, true>(bg, c, px, py, pz, bpm,
             [&](uint32_t, const float4&, float, float, float, float l2) {
                 hit |= l2 <= r2 ? 1u : 0u;
             });

@@ -236,7 +236,7 @@ void solver_step(reyn_solver& sv, reyn_particles& st, const Grid& grid,
 // neighbours within r (self included) + sum_b m_b W_ib over the boundary
 // samples, per grid slot over packed points; `owner` maps a slot back to
 // the caller's index on a grid built without reorder
-template <int KIND, int R>
+template <int KIND, int R, bool XYZ>
 __global__ void __launch_bounds__(NBR_THREADS) k_compute_densities(uint32_t n, GridView g,
     KernelConst kc, const float4* __restrict__ pts, const uint32_t* __restrict__ owner, Bdy b,
     float* __restrict__ rho, uint32_t* __restrict__ status)
@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(NBR_THREADS) k_compute_densities(uint32_t n, G
         c = clamp_cell(g, c, R);
     }
     float rf = 0.f;
-    for_each_neighbour<R>(g, c, me.x, me.y, me.z, pts,
+    for_each_neighbour<R, XYZ>(g, c, me.x, me.y, me.z, pts,
         [&](uint32_t, const float4& q, float, float, float, float l2) {
             rf += q.w * pair_w<KIND>(kc, l2);
         });
@@ -291,12 +291,11 @@ void compute_densities(const Grid& g, const float* x, const float* y, const floa
     uint32_t* st = const_cast<uint32_t*>(g.status.get());
     auto go = [&](auto K) {
         constexpr int KIND = decltype(K)::value;
-        if (g.geom.range == 2)
-            k_compute_densities<KIND, 2><<<nb, NBR_THREADS, 0, s>>>(n, v, kc, pts.get(), order, b,
-                rho, st);
-        else
-            k_compute_densities<KIND, 1><<<nb, NBR_THREADS, 0, s>>>(n, v, kc, pts.get(), order, b,
-                rho, st);
+        const bool xyz = g.geom.order == REYN_ORDER_XYZ;
+        auto kern = g.geom.range == 2
+            ? (xyz ? k_compute_densities<KIND, 2, true> : k_compute_densities<KIND, 2, false>)
+            : (xyz ? k_compute_densities<KIND, 1, true> : k_compute_densities<KIND, 1, false>);
+        kern<<<nb, NBR_THREADS, 0, s>>>(n, v, kc, pts.get(), order, b, rho, st);
     };
     ProfScope scope("k_compute_densities", s);
     switch (kind) {
