@@ -1056,12 +1056,14 @@ k_density(uint32_t n, Fluid f, Bdy b,
 
 // write_non_prs_acc_ff (solver.cuh:40-69): gravity + artificial viscosity;
 // optionally fused with integrate_a_v_only (solver.cu:3-13) into vel_out
-// (and its FP16 copy velh_out under mixed precision)
+// (and its FP16 copy velh_out under mixed precision). With p_old (IISPH) the
+// fourth component of vel_out is m p_old, which the diagonal pass reads with
+// the neighbour's velocity.
 template <int KIND, int R, int MIX, bool BATCH>
 __device__ __forceinline__ void nonpressure(uint32_t n, const Fluid& f,
     const float4* __restrict__ vel, const uint2* __restrict__ velh, float nu10, float eps,
     float3 grav, float dt, float4* __restrict__ acc, float4* __restrict__ vel_out,
-    uint2* __restrict__ velh_out)
+    uint2* __restrict__ velh_out, const float* __restrict__ p_old)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
@@ -1082,7 +1084,7 @@ __device__ __forceinline__ void nonpressure(uint32_t n, const Fluid& f,
     acc[i] = make_float4(ax, ay, az, 0.f);
     if (vel_out) {
         const float4 vs = make_float4(vi.x + dt * ax, vi.y + dt * ay, vi.z + dt * az, vi.w);
-        vel_out[i] = vs;
+        vel_out[i] = make_float4(vs.x, vs.y, vs.z, p_old ? me.w * p_old[i] : vs.w);
         if constexpr (MIX)
             velh_out[i] = float4_to_half4(vs);
     }
@@ -1266,14 +1268,25 @@ __global__ void k_advect(uint32_t n, const float4* __restrict__ pm,
     tail_reduce(tail, vn);
 }
 
-// _compute_diagonal_elem_and_source_term (IISPH.cu:11-66) + warm start
-// (IISPH.cu:193-209)
+// The pressure passes of FP32 and MIXED read the neighbours' positions and
+// pressures as one record xq = (x, y, z, m p), with the gradient moment
+// G_i = sum_j m_j grad W_ij + g_b (gq) of the diagonal pass:
+//   sum_j m_j (p_i + p_j) grad W_ij + p_i g_b = p_i G_i + sum_j (m_j p_j) grad W_ij
+// They are bound by the L1's gathers (a warp's 16-byte gather takes 8 to 16
+// wavefronts, a 4-byte one of p_j another 2 to 8), so one gather a pair
+// instead of two pays: pressure accelerations 92 -> 77 us, diagonal pass 150
+// -> 135, final pass 100 -> 85 (1M particles, FP32, developed flow; 66 -> 60,
+// 114 -> 97, 74 -> 67 from rest). The Jacobi sweep keeps its differences
+// a_i - a_j, which are exact where the accelerations are nearly uniform.
+
+// _compute_diagonal_elem_and_source_term (IISPH.cu:11-66) without warm start
+// (IISPH.cu:193-209); writes G and the record of the pressure it starts from
 template <int KIND, int R, int MIX = 0, bool BATCH = false, int MB = NBR_THREADS>
 __global__ void __launch_bounds__(MB) k_iisph_diag(uint32_t n, Fluid f,
     const float4* __restrict__ vel, const uint2* __restrict__ velh,
-    const float4* __restrict__ bterm, float rho0, float dt,
-    float omega, int warmstart, float tiny, float* __restrict__ aii, float* __restrict__ sii,
-    float* __restrict__ p)
+    const float4* __restrict__ bterm, const float* __restrict__ rho, float rho0, float dt,
+    float omega, float tiny, float* __restrict__ aii, float* __restrict__ sii,
+    float* __restrict__ p, float4* __restrict__ gq, float4* __restrict__ xq)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
@@ -1305,24 +1318,28 @@ __global__ void __launch_bounds__(MB) k_iisph_diag(uint32_t n, Fluid f,
     gz += bt.z;
     const float gss = fmaf(gx, gx, fmaf(gy, gy, gz * gz));
     const float a = -dt * (gss + me.w * gsq) / (rho0 * rho0);
-    const float s = (rho0 - vi.w) / dt - (vdiv + fmaf(vi.x, bt.x, fmaf(vi.y, bt.y, vi.z * bt.z)));
+    const float s = (rho0 - rho[i]) / dt - (vdiv + fmaf(vi.x, bt.x, fmaf(vi.y, bt.y, vi.z * bt.z)));
     aii[i] = a;
     sii[i] = s;
-    p[i] = warmstart ? p[i] * 0.5f : jacobi_update(omega, a, 0.f, s, tiny);
+    gq[i] = make_float4(gx, gy, gz, 0.f);
+    const float pn = jacobi_update(omega, a, 0.f, s, tiny);
+    p[i] = pn;
+    xq[i] = make_float4(me.x, me.y, me.z, me.w * pn);
 }
 
-// the diagonal pass fused with the first sweep's pressure accelerations
-// under the warm start: every neighbour's warm-started pressure is half its
-// carried pressure, so a_i = -(1/rho0^2)(sum m_j (p_i' + p_j') grad W_ij +
-// p_i' g_b) with p' = 0.5 p can be summed in the same neighbour loop. p_old
-// is read, p_new written (p_new = 0.5 p_old).
+// the diagonal pass fused with the warm start and the first sweep's pressure
+// accelerations: every neighbour's warm-started pressure is half its carried
+// pressure, so a_i = -(1/rho0^2)(p_i' G_i + sum m_j p_j' grad W_ij) with
+// p' = 0.5 p is summed in the same neighbour loop. p_old is read, p_new
+// written (p_new = 0.5 p_old). FP32: m_j p_j comes with the neighbour's
+// velocity (its fourth component).
 template <int KIND, int R, int MIX = 0, bool BATCH = false, int MB = NBR_THREADS>
 __global__ void __launch_bounds__(MB) k_iisph_diag_pacc(uint32_t n, Fluid f,
     const float4* __restrict__ vel, const uint2* __restrict__ velh,
-    const float4* __restrict__ bterm, float rho0, float dt,
+    const float4* __restrict__ bterm, const float* __restrict__ rho, float rho0, float dt,
     float r0i, const float* __restrict__ p_old, float* __restrict__ aii,
-    float* __restrict__ sii, float* __restrict__ p_new, float4* __restrict__ acc,
-    uint2* __restrict__ acch_out)
+    float* __restrict__ sii, float* __restrict__ p_new, float4* __restrict__ gq,
+    float4* __restrict__ acc, uint2* __restrict__ acch_out)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
@@ -1332,11 +1349,11 @@ __global__ void __launch_bounds__(MB) k_iisph_diag_pacc(uint32_t n, Fluid f,
     const float pi = p_old[i] * 0.5f;
     float gx = 0.f, gy = 0.f, gz = 0.f, vdiv = 0.f, gsq = 0.f;
     [[maybe_unused]] Kahan vk; // mixed modes: compensated divergence sum
-    float ax = 0.f, ay = 0.f, az = 0.f;
+    float sx = 0.f, sy = 0.f, sz = 0.f;
     for_each_listed<R, MIX, false, BATCH>(f, i, me,
         [&](uint32_t j, const float4& q, float dx, float dy, float dz, float l2) {
             const float4 vj = nbr_vel<MIX>(vel, velh, j);
-            const float pj = __ldg(p_old + j) * 0.5f;
+            const float mp = MIX ? q.w * __ldg(p_old + j) : vj.w;
             const float g = pair_g<KIND>(f.kc, l2);
             const float mg = q.w * g;
             gx += mg * dx;
@@ -1348,32 +1365,47 @@ __global__ void __launch_bounds__(MB) k_iisph_diag_pacc(uint32_t n, Fluid f,
             else
                 vdiv += dv;
             gsq += mg * g * l2;
-            const float sp = q.w * (pi + pj) * g;
-            ax += sp * dx;
-            ay += sp * dy;
-            az += sp * dz;
+            const float sp = mp * g;
+            sx += sp * dx;
+            sy += sp * dy;
+            sz += sp * dz;
         });
     if constexpr (MIX)
         vdiv = vk.sum;
     const float4 bt = bterm[i];
-    const float4 ai = make_float4(-r0i * (ax + pi * bt.x), -r0i * (ay + pi * bt.y),
-        -r0i * (az + pi * bt.z), 0.f);
-    acc[i] = ai;
-    if constexpr (MIX)
-        acch_out[i] = pack_acc(ai.x, ai.y, ai.z);
     gx += bt.x;
     gy += bt.y;
     gz += bt.z;
+    gq[i] = make_float4(gx, gy, gz, 0.f);
+    const float4 ai = make_float4(-r0i * fmaf(pi, gx, 0.5f * sx), -r0i * fmaf(pi, gy, 0.5f * sy),
+        -r0i * fmaf(pi, gz, 0.5f * sz), 0.f);
+    acc[i] = ai;
+    if constexpr (MIX)
+        acch_out[i] = pack_acc(ai.x, ai.y, ai.z);
     const float gss = fmaf(gx, gx, fmaf(gy, gy, gz * gz));
     aii[i] = -dt * (gss + me.w * gsq) / (rho0 * rho0);
-    sii[i] = (rho0 - vi.w) / dt - (vdiv + fmaf(vi.x, bt.x, fmaf(vi.y, bt.y, vi.z * bt.z)));
+    sii[i] = (rho0 - rho[i]) / dt - (vdiv + fmaf(vi.x, bt.x, fmaf(vi.y, bt.y, vi.z * bt.z)));
     p_new[i] = pi;
 }
 
-// _set_pressure_accelerations (IISPH.cu:68-98)
+// _set_pressure_accelerations (IISPH.cu:68-98); f.pm is xq
+template <int KIND, int R, int MIX, bool BATCH>
+__device__ __forceinline__ float3 pressure_sum(const Fluid& f, uint32_t i, const float4& me)
+{
+    float sx = 0.f, sy = 0.f, sz = 0.f;
+    for_each_listed<R, MIX, false, BATCH>(f, i, me,
+        [&](uint32_t, const float4& q, float dx, float dy, float dz, float l2) {
+            const float s = q.w * pair_g<KIND>(f.kc, l2);
+            sx += s * dx;
+            sy += s * dy;
+            sz += s * dz;
+        });
+    return make_float3(sx, sy, sz);
+}
+
 template <int KIND, int R, int MIX, bool BATCH>
 __device__ __forceinline__ void iisph_pacc(uint32_t i, uint32_t n, const Fluid& f,
-    const float* __restrict__ p, const float4* __restrict__ bterm, float r0i,
+    const float* __restrict__ p, const float4* __restrict__ gq, float r0i,
     float4* __restrict__ acc, uint2* __restrict__ acch_out, const uint32_t* __restrict__ gate)
 {
     // a captured step's loop body: the first sweep uses the accelerations of
@@ -1385,18 +1417,11 @@ __device__ __forceinline__ void iisph_pacc(uint32_t i, uint32_t n, const Fluid& 
             return;
     }
     const float4 me = f.pm[i];
+    const float3 s = pressure_sum<KIND, R, MIX, BATCH>(f, i, me);
     const float pi = p[i];
-    float ax = 0.f, ay = 0.f, az = 0.f;
-    for_each_listed<R, MIX, false, BATCH>(f, i, me,
-        [&](uint32_t j, const float4& q, float dx, float dy, float dz, float l2) {
-            const float s = q.w * (pi + __ldg(p + j)) * pair_g<KIND>(f.kc, l2);
-            ax += s * dx;
-            ay += s * dy;
-            az += s * dz;
-        });
-    const float4 bt = bterm[i];
-    const float4 ai = make_float4(-r0i * (ax + pi * bt.x), -r0i * (ay + pi * bt.y),
-        -r0i * (az + pi * bt.z), 0.f);
+    const float4 G = gq[i];
+    const float4 ai = make_float4(-r0i * fmaf(pi, G.x, s.x), -r0i * fmaf(pi, G.y, s.y),
+        -r0i * fmaf(pi, G.z, s.z), 0.f);
     acc[i] = ai;
     if constexpr (MIX)
         acch_out[i] = pack_acc(ai.x, ai.y, ai.z);
@@ -1409,7 +1434,7 @@ template <int KIND, int R, int MIX, bool BATCH>
 __device__ __forceinline__ void iisph_jacobi(uint32_t i, uint32_t n, const Fluid& f,
     const float4* __restrict__ acc, const float4* __restrict__ bterm,
     const float* __restrict__ aii, const float* __restrict__ sii, float* __restrict__ p,
-    float dt, float omega, float tiny, float thr, SweepStats* stats)
+    float4* __restrict__ xq, float dt, float omega, float tiny, float thr, SweepStats* stats)
 {
     unsigned over = 0;
     double epos = 0.0;
@@ -1448,7 +1473,9 @@ __device__ __forceinline__ void iisph_jacobi(uint32_t i, uint32_t n, const Fluid
         const float4 bt = bterm[i];
         const float Ap = dt * (sum + fmaf(ai.x, bt.x, fmaf(ai.y, bt.y, ai.z * bt.z)));
         const float s = sii[i];
-        p[i] = p[i] + jacobi_update(omega, aii[i], Ap, s, tiny);
+        const float pn = p[i] + jacobi_update(omega, aii[i], Ap, s, tiny);
+        p[i] = pn;
+        xq[i] = make_float4(me.x, me.y, me.z, me.w * pn);
         const float err = (Ap - s) * dt;
         over = err > thr ? 1u : 0u;
         epos = err > 0.f ? (double)err : 0.0;
@@ -1462,10 +1489,10 @@ __device__ __forceinline__ void iisph_jacobi(uint32_t i, uint32_t n, const Fluid
 
 template <int KIND, int R, int MIX = 0, bool BATCH = false, int MB = NBR_THREADS>
 __global__ void __launch_bounds__(MB) k_iisph_pacc(uint32_t n, Fluid f,
-    const float* __restrict__ p, const float4* __restrict__ bterm, float r0i,
+    const float* __restrict__ p, const float4* __restrict__ gq, float r0i,
     float4* __restrict__ acc, uint2* __restrict__ acch_out, const uint32_t* __restrict__ gate)
 {
-    iisph_pacc<KIND, R, MIX, BATCH>(blockIdx.x * blockDim.x + threadIdx.x, n, f, p, bterm, r0i,
+    iisph_pacc<KIND, R, MIX, BATCH>(blockIdx.x * blockDim.x + threadIdx.x, n, f, p, gq, r0i,
         acc, acch_out, gate);
 }
 
@@ -1473,19 +1500,19 @@ template <int KIND, int R, int MIX = 0, bool BATCH = false, int MB = NBR_THREADS
 __global__ void __launch_bounds__(MB) k_iisph_jacobi(uint32_t n, Fluid f,
     const float4* __restrict__ acc, const float4* __restrict__ bterm,
     const float* __restrict__ aii, const float* __restrict__ sii, float* __restrict__ p,
-    float dt, float omega, float tiny, float thr, SweepStats* stats)
+    float4* __restrict__ xq, float dt, float omega, float tiny, float thr, SweepStats* stats)
 {
     iisph_jacobi<KIND, R, MIX, BATCH>(blockIdx.x * blockDim.x + threadIdx.x, n, f, acc, bterm,
-        aii, sii, p, dt, omega, tiny, thr, stats);
+        aii, sii, p, xq, dt, omega, tiny, thr, stats);
 }
 
 template <int KIND, int R, int MIX, int MB>
 __global__ void __launch_bounds__(MB) k_iisph_pacc_tiles(uint32_t n, Fluid f,
-    const float* __restrict__ p, const float4* __restrict__ bterm, float r0i,
+    const float* __restrict__ p, const float4* __restrict__ gq, float r0i,
     float4* __restrict__ acc, uint2* __restrict__ acch_out, const uint32_t* __restrict__ gate,
     Tiles tl)
 {
-    REYN_TILE_LOOP(tl, (iisph_pacc<KIND, R, MIX, true>(i, n, f, p, bterm, r0i, acc, acch_out,
+    REYN_TILE_LOOP(tl, (iisph_pacc<KIND, R, MIX, true>(i, n, f, p, gq, r0i, acc, acch_out,
         gate)));
 }
 
@@ -1493,10 +1520,11 @@ template <int KIND, int R, int MIX, int MB>
 __global__ void __launch_bounds__(MB) k_iisph_jacobi_tiles(uint32_t n, Fluid f,
     const float4* __restrict__ acc, const float4* __restrict__ bterm,
     const float* __restrict__ aii, const float* __restrict__ sii, float* __restrict__ p,
-    float dt, float omega, float tiny, float thr, SweepStats* stats, Tiles tl)
+    float4* __restrict__ xq, float dt, float omega, float tiny, float thr, SweepStats* stats,
+    Tiles tl)
 {
-    REYN_TILE_LOOP(tl, (iisph_jacobi<KIND, R, MIX, true>(i, n, f, acc, bterm, aii, sii, p, dt,
-        omega, tiny, thr, stats)));
+    REYN_TILE_LOOP(tl, (iisph_jacobi<KIND, R, MIX, true>(i, n, f, acc, bterm, aii, sii, p, xq,
+        dt, omega, tiny, thr, stats)));
 }
 
 // The mixed modes' sweep kernels for one scene and the polynomial kernels,
@@ -1510,10 +1538,10 @@ constexpr bool occupancy_variant = MIX != 0 && KIND != K_COS;
 
 template <int KIND, int R, int MIX, int MB>
 __global__ void __launch_bounds__(MB, (65536 / 40) / MB) k_iisph_pacc_occ(uint32_t n, Fluid f,
-    const float* __restrict__ p, const float4* __restrict__ bterm, float r0i,
+    const float* __restrict__ p, const float4* __restrict__ gq, float r0i,
     float4* __restrict__ acc, uint2* __restrict__ acch_out, const uint32_t* __restrict__ gate)
 {
-    iisph_pacc<KIND, R, MIX, false>(blockIdx.x * blockDim.x + threadIdx.x, n, f, p, bterm, r0i,
+    iisph_pacc<KIND, R, MIX, false>(blockIdx.x * blockDim.x + threadIdx.x, n, f, p, gq, r0i,
         acc, acch_out, gate);
 }
 
@@ -1521,10 +1549,10 @@ template <int KIND, int R, int MIX, int MB>
 __global__ void __launch_bounds__(MB, (65536 / 40) / MB) k_iisph_jacobi_occ(uint32_t n, Fluid f,
     const float4* __restrict__ acc, const float4* __restrict__ bterm,
     const float* __restrict__ aii, const float* __restrict__ sii, float* __restrict__ p,
-    float dt, float omega, float tiny, float thr, SweepStats* stats)
+    float4* __restrict__ xq, float dt, float omega, float tiny, float thr, SweepStats* stats)
 {
     iisph_jacobi<KIND, R, MIX, false>(blockIdx.x * blockDim.x + threadIdx.x, n, f, acc, bterm,
-        aii, sii, p, dt, omega, tiny, thr, stats);
+        aii, sii, p, xq, dt, omega, tiny, thr, stats);
 }
 
 // a batch's sweeps: persistent launches over the active tiles (tl)
@@ -1564,20 +1592,21 @@ void launch_iisph_jacobi(unsigned nb, unsigned bs, cudaStream_t q, Tiles tl, boo
 
 #define REYN_NONPRESSURE_ARGS uint32_t n, Fluid f, const float4* __restrict__ vel, \
     const uint2* __restrict__ velh, float nu10, float eps, float3 grav, float dt, \
-    float4* __restrict__ acc, float4* __restrict__ vel_out, uint2* __restrict__ velh_out
+    float4* __restrict__ acc, float4* __restrict__ vel_out, uint2* __restrict__ velh_out, \
+    const float* __restrict__ p_old
 
 template <int KIND, int R, int MIX = 0, bool BATCH = false, int MB = NBR_THREADS>
 __global__ void __launch_bounds__(MB) k_nonpressure(REYN_NONPRESSURE_ARGS)
 {
     nonpressure<KIND, R, MIX, BATCH>(n, f, vel, velh, nu10, eps, grav, dt, acc, vel_out,
-        velh_out);
+        velh_out, p_old);
 }
 
 template <int KIND, int R, int MIX, int MB>
 __global__ void __launch_bounds__(MB, (65536 / 48) / MB) k_nonpressure_occ(REYN_NONPRESSURE_ARGS)
 {
     nonpressure<KIND, R, MIX, false>(n, f, vel, velh, nu10, eps, grav, dt, acc, vel_out,
-        velh_out);
+        velh_out, p_old);
 }
 
 #undef REYN_NONPRESSURE_ARGS
@@ -1601,7 +1630,7 @@ void launch_nonpressure(unsigned nb, unsigned bs, cudaStream_t q, A... a)
 // accelerations go straight to the solver's SoA arrays
 template <int KIND, int R, int MIX = 0, bool BATCH = false, int MB = NBR_THREADS>
 __global__ void __launch_bounds__(MB) k_iisph_final(uint32_t n, Fluid f,
-    const float* __restrict__ p, const float4* __restrict__ bterm, float r0i,
+    const float* __restrict__ p, const float4* __restrict__ gq, float r0i,
     const float4* __restrict__ vel, float dt, Soa3 acc,
     float* __restrict__ x, float* __restrict__ y, float* __restrict__ z,
     float* __restrict__ vx, float* __restrict__ vy, float* __restrict__ vz, Tail tail)
@@ -1610,19 +1639,12 @@ __global__ void __launch_bounds__(MB) k_iisph_final(uint32_t n, Fluid f,
     float vn = 0.f;
     if (i < n) {
     const float4 me = f.pm[i];
+    const float3 s = pressure_sum<KIND, R, MIX, BATCH>(f, i, me);
     const float pi = p[i];
-    float ax = 0.f, ay = 0.f, az = 0.f;
-    for_each_listed<R, MIX, false, BATCH>(f, i, me,
-        [&](uint32_t j, const float4& q, float dx, float dy, float dz, float l2) {
-            const float s = q.w * (pi + __ldg(p + j)) * pair_g<KIND>(f.kc, l2);
-            ax += s * dx;
-            ay += s * dy;
-            az += s * dz;
-        });
-    const float4 bt = bterm[i];
-    ax = -r0i * (ax + pi * bt.x);
-    ay = -r0i * (ay + pi * bt.y);
-    az = -r0i * (az + pi * bt.z);
+    const float4 G = gq[i];
+    const float ax = -r0i * fmaf(pi, G.x, s.x);
+    const float ay = -r0i * fmaf(pi, G.y, s.y);
+    const float az = -r0i * fmaf(pi, G.z, s.z);
     acc.x[i] = ax;
     acc.y[i] = ay;
     acc.z[i] = az;
@@ -1886,6 +1908,10 @@ void solver_step_t(reyn_solver& sv, reyn_particles& st, const Grid& grid,
     uint4* REC0 = rec16 ? sv.rec0.get() : nullptr;
     uint4* REC1 = rec16 ? sv.rec1.get() : nullptr;
     f.acch = ACH;
+    // FP32 and MIXED: the pressure passes' records (x, y, z, m p) in place of
+    // (x, y, z, m)
+    Fluid fq = f;
+    fq.pm = sv.xq.get();
     auto body = [&](auto KC, auto RC, auto MC, auto BC) {
         constexpr int K = decltype(KC)::value;
         constexpr int R = decltype(RC)::value;
@@ -1919,7 +1945,7 @@ void solver_step_t(reyn_solver& sv, reyn_particles& st, const Grid& grid,
             REYN_KERNEL("k_nonpressure", s,
                 launch_nonpressure<K, R, 0, B, MB>(nb, bs, s, n, f, (const float4*)st.vel.get(),
                 (const uint2*)nullptr, nu10, eps, grav, dt, sv.acc.get(), sv.vel2.get(),
-                (uint2*)nullptr));
+                (uint2*)nullptr, (const float*)nullptr));
             float4* v = sv.vel2.get();
             // one PCISPH iteration: prediction and pressure (a batch: over
             // the tiles of the scenes still iterating)
@@ -2094,24 +2120,25 @@ void solver_step_t(reyn_solver& sv, reyn_particles& st, const Grid& grid,
         } else { // IISPH
             REYN_KERNEL("k_nonpressure", s,
                 launch_nonpressure<K, R, MIX, B, MB>(nb, bs, s, n, f, (const float4*)st.vel.get(),
-                (const uint2*)VH, nu10, eps, grav, dt, sv.acc.get(), sv.vel2.get(), VH2));
+                (const uint2*)VH, nu10, eps, grav, dt, sv.acc.get(), sv.vel2.get(), VH2,
+                (const float*)sv.p.get()));
             const float tiny = tiny_threshold();
             auto pacc = [&] {
                 REYN_KERNEL("k_iisph_pacc", s,
-                    launch_iisph_pacc<K, R, MIX, B, MB>(nb, bs, s, tl, persist, n, f, sv.p.get(),
-                    sv.bterm.get(), r0i, sv.acc.get(), ACH, (const uint32_t*)nullptr));
+                    launch_iisph_pacc<K, R, MIX, B, MB>(nb, bs, s, tl, persist, n, fq, sv.p.get(),
+                    sv.gq.get(), r0i, sv.acc.get(), ACH, (const uint32_t*)nullptr));
             };
             if (P.warmstart) {
                 REYN_KERNEL("k_iisph_diag_pacc", s,
                     k_iisph_diag_pacc<K, R, MIX, B, MB><<<nb, bs, 0, s>>>(n, f, sv.vel2.get(),
-                    VH2, sv.bterm.get(), rho0, dt, r0i, sv.p.get(), sv.aii.get(), sv.sii.get(),
-                    sv.p_tmp.get(), sv.acc.get(), ACH));
+                    VH2, sv.bterm.get(), sv.rho.get(), rho0, dt, r0i, sv.p.get(), sv.aii.get(),
+                    sv.sii.get(), sv.p_tmp.get(), sv.gq.get(), sv.acc.get(), ACH));
                 sv.p.swap(sv.p_tmp);
             } else {
                 REYN_KERNEL("k_iisph_diag", s,
                     k_iisph_diag<K, R, MIX, B, MB><<<nb, bs, 0, s>>>(n, f, sv.vel2.get(),
-                    VH2, sv.bterm.get(), rho0, dt, P.omega, P.warmstart, tiny, sv.aii.get(),
-                    sv.sii.get(), sv.p.get()));
+                    VH2, sv.bterm.get(), sv.rho.get(), rho0, dt, P.omega, tiny, sv.aii.get(),
+                    sv.sii.get(), sv.p.get(), sv.gq.get(), sv.xq.get()));
                 pacc();
             }
             const float thr = P.eta * rho0;
@@ -2122,14 +2149,14 @@ void solver_step_t(reyn_solver& sv, reyn_particles& st, const Grid& grid,
                 graph_loop([&](cudaStream_t q, cudaGraphConditionalHandle h) {
                     SweepStats* slot = ns ? scene_slot : slots;
                     REYN_KERNEL("k_iisph_pacc", q,
-                        launch_iisph_pacc<K, R, MIX, B, MB>(nb, bs, q, tl, persist, n, f, sv.p.get(),
-                        sv.bterm.get(), r0i, sv.acc.get(), ACH, (const uint32_t*)gx->gate));
+                        launch_iisph_pacc<K, R, MIX, B, MB>(nb, bs, q, tl, persist, n, fq, sv.p.get(),
+                        sv.gq.get(), r0i, sv.acc.get(), ACH, (const uint32_t*)gx->gate));
                     REYN_CUDA(cudaMemsetAsync(slot, 0, sizeof(SweepStats) * (ns ? ns : 1), q));
                     REYN_KERNEL("k_iisph_jacobi", q,
                         launch_iisph_jacobi<K, R, MIX, B, MB>(nb, bs, q, tl, persist, n, f,
                         (const float4*)sv.acc.get(), (const float4*)sv.bterm.get(),
-                        (const float*)sv.aii.get(), (const float*)sv.sii.get(), sv.p.get(), dt,
-                        P.omega, tiny, thr, slot));
+                        (const float*)sv.aii.get(), (const float*)sv.sii.get(), sv.p.get(),
+                        sv.xq.get(), dt, P.omega, tiny, thr, slot));
                     if (ns)
                         scene_converge_dev(q, P.convergence == REYN_CONV_AVERAGE ? 1 : 2);
                     decide(q, h, slot);
@@ -2143,8 +2170,8 @@ void solver_step_t(reyn_solver& sv, reyn_particles& st, const Grid& grid,
                 REYN_KERNEL("k_iisph_jacobi", s,
                     launch_iisph_jacobi<K, R, MIX, B, MB>(nb, bs, s, tl, persist, n, f,
                     (const float4*)sv.acc.get(), (const float4*)sv.bterm.get(),
-                    (const float*)sv.aii.get(), (const float*)sv.sii.get(), sv.p.get(), dt,
-                    P.omega, tiny, thr, slot));
+                    (const float*)sv.aii.get(), (const float*)sv.sii.get(), sv.p.get(),
+                    sv.xq.get(), dt, P.omega, tiny, thr, slot));
                 iters += 1;
                 const bool last = max_it && iters >= max_it;
                 if (iters < P.min_iter && !last) {
@@ -2176,7 +2203,7 @@ void solver_step_t(reyn_solver& sv, reyn_particles& st, const Grid& grid,
                 pacc();
             }
             REYN_KERNEL("k_iisph_final", s,
-                k_iisph_final<K, R, MIX, B, MB><<<nb, bs, 0, s>>>(n, f, sv.p.get(), sv.bterm.get(),
+                k_iisph_final<K, R, MIX, B, MB><<<nb, bs, 0, s>>>(n, fq, sv.p.get(), sv.gq.get(),
                 r0i, sv.vel2.get(), dt, Soa3 { sv.ax.get(), sv.ay.get(), sv.az.get() }, X, Y, Z,
                 VX, VY, VZ, tail));
         }

@@ -77,7 +77,11 @@ void ensure_buffers(reyn_solver& sv, uint32_t n)
     } else if (sv.prm.precision == REYN_PRECISION_MIXED_POS16) {
         sv.rec0.resize(n);
         sv.rec1.resize(n);
+    }
+    if (sv.scheme == REYN_IISPH) {
         sv.gq.resize(n);
+        if (sv.prm.precision != REYN_PRECISION_MIXED_POS16)
+            sv.xq.resize(n);
     }
     if (sv.p.size() != n) {
         sv.p.resize(n);
