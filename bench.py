@@ -70,7 +70,6 @@ ALG_BYTES = {
     "k_gather": 4 + 28 + 28 + 32,     # perm, 7 arrays in/out, packed copies
     "k_vmax": 12,
     "k_bounds_enforce": 24 + 12,
-    "k_unpack_acc": 16 + 12,
 }
 
 

@@ -69,6 +69,24 @@ struct Fluid {
     const uint8_t* __restrict__ active;
 };
 
+// Log2 of the particles a warp of the density pass works on. A small state
+// leaves the SMs short of warps, and each waits out the union of its lanes'
+// cell rows and every latency in turn; it is spread over more warps with
+// fewer particles in their first lanes (the same arithmetic per particle)
+// until there are WARP_TARGET of them, about 3.5 a scheduler. Measured on whole
+// steps: 8k particles (PCISPH, captured) 167 -> 160 us, 16k (SESPH) 148 -> 140,
+// 32k 152 -> 151; a target of 4096 costs at 64k (274 -> 295). The list passes,
+// whose lanes all take the same rounds, only lose by it.
+constexpr uint32_t WARP_TARGET = 2048;
+
+inline uint32_t warp_shift(uint32_t n)
+{
+    uint32_t s = 5;
+    while (s > 2 && (n >> s) < WARP_TARGET)
+        --s;
+    return s;
+}
+
 // ---- mixed precision ----------------------------------------------------------
 // MIXED_POS16 records are 16 bytes: each position coordinate as a 16-bit
 // wrapped fixed-point number, the position in cells modulo 4 at a resolution
@@ -997,7 +1015,8 @@ unsigned persistent_grid(Kern kern, unsigned bs, unsigned tiles)
 // neighbour list, written entry by entry (a block's rows form one 32 KB
 // region, so the L2 merges the scattered 4-byte stores into full lines).
 // MIXED: the particle's FP16 velocity/density record is written for later
-// passes; MIXED_POS16: its 16-byte record for the non-pressure pass.
+// passes; MIXED_POS16: its 16-byte record for the non-pressure pass. inv_rho
+// (SESPH): vel.w receives 1 / rho instead of rho. shift: warp_shift(n).
 // Bound by instruction issue (the cell traversal). One scene: held to 40
 // registers (12 blocks of 128 per SM); 48 registers run slower (514 against
 // 502 us on the 4M dam break in MIXED_POS16), 32 as well (527).
@@ -1005,9 +1024,10 @@ template <int KIND, int R, bool XYZ, int MIX = 0, bool BATCH = false, int MB = N
 __global__ void __launch_bounds__(MB, (BATCH ? 0 : 65536 / 40 / MB))
 k_density(uint32_t n, Fluid f, Bdy b,
     float* __restrict__ rho, float4* __restrict__ vel, float4* __restrict__ bterm,
-    uint4* __restrict__ rec_out, uint2* __restrict__ velh_out)
+    uint4* __restrict__ rec_out, uint2* __restrict__ velh_out, bool inv_rho, uint32_t shift)
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t i = (t & 31u) >> shift ? n : ((t >> 5) << shift) + (t & 31u);
     const bool valid = i < n; // the boundary sums need the whole warp
     const float4 me = valid ? f.pm[i] : make_float4(0.f, 0.f, 0.f, 0.f);
     uint32_t scene = 0;
@@ -1041,7 +1061,7 @@ k_density(uint32_t n, Fluid f, Bdy b,
         rf = rk.sum;
     const float r = rf + reinterpret_cast<const volatile float*>(bterm + i)[3];
     rho[i] = r;
-    vel[i].w = r;
+    vel[i].w = inv_rho ? 1.f / r : r;
     f.ncount[i] = cnt;
     if constexpr (MIX == MIX_POS16) {
         const float4 v = vel[i];
@@ -1054,16 +1074,16 @@ k_density(uint32_t n, Fluid f, Bdy b,
     }
 }
 
-// write_non_prs_acc_ff (solver.cuh:40-69): gravity + artificial viscosity;
-// optionally fused with integrate_a_v_only (solver.cu:3-13) into vel_out
-// (and its FP16 copy velh_out under mixed precision). With p_old (IISPH) the
+// write_non_prs_acc_ff (solver.cuh:40-69): gravity + artificial viscosity,
+// fused with integrate_a_v_only (solver.cu:3-13) into vel_out (and its FP16
+// copy velh_out under mixed precision). With p_old (IISPH) the
 // fourth component of vel_out is m p_old, which the diagonal pass reads with
 // the neighbour's velocity.
 template <int KIND, int R, int MIX, bool BATCH>
 __device__ __forceinline__ void nonpressure(uint32_t n, const Fluid& f,
     const float4* __restrict__ vel, const uint2* __restrict__ velh, float nu10, float eps,
-    float3 grav, float dt, float4* __restrict__ acc, float4* __restrict__ vel_out,
-    uint2* __restrict__ velh_out, const float* __restrict__ p_old)
+    float3 grav, float dt, float4* __restrict__ vel_out, uint2* __restrict__ velh_out,
+    const float* __restrict__ p_old)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
@@ -1081,26 +1101,27 @@ __device__ __forceinline__ void nonpressure(uint32_t n, const Fluid& f,
             ay += s * dy;
             az += s * dz;
         });
-    acc[i] = make_float4(ax, ay, az, 0.f);
-    if (vel_out) {
-        const float4 vs = make_float4(vi.x + dt * ax, vi.y + dt * ay, vi.z + dt * az, vi.w);
-        vel_out[i] = make_float4(vs.x, vs.y, vs.z, p_old ? me.w * p_old[i] : vs.w);
-        if constexpr (MIX)
-            velh_out[i] = float4_to_half4(vs);
-    }
+    const float4 vs = make_float4(vi.x + dt * ax, vi.y + dt * ay, vi.z + dt * az, vi.w);
+    vel_out[i] = make_float4(vs.x, vs.y, vs.z, p_old ? me.w * p_old[i] : vs.w);
+    if constexpr (MIX)
+        velh_out[i] = float4_to_half4(vs);
 }
 
-__device__ __forceinline__ float eos_sesph(float rho, float k, float rho0)
+// p / rho^2 of SESPH's equation of state p = max(0, k (rho / rho0 - 1))
+// (SESPH.cu:6-12) from 1 / rho: (k / rho0) (1 / rho) (1 - rho0 / rho)
+__device__ __forceinline__ float pressure_term_sesph(float rho_inv, float k_r0, float rho0)
 {
-    return fmaxf(0.f, k * (rho / rho0 - 1.f)); // SESPH.cu:6-12
+    return fmaxf(0.f, k_r0 * rho_inv * fmaf(-rho0, rho_inv, 1.f));
 }
 
 // _compute_accelerations (SESPH.cu:15-65) fused with integrate (solver.cu:
-// 15-32): writes the new SoA state
+// 15-32): writes the new SoA state and the accelerations. vel.w is 1 / rho,
+// formed once per particle by the density pass: one division a pair instead
+// of the four that rho needs (a step of 1M particles 546 -> 497 us).
 template <int KIND, int R, bool BATCH = false, int MB = NBR_THREADS>
 __global__ void __launch_bounds__(MB) k_sesph(uint32_t n, Fluid f,
-    const float4* __restrict__ vel, const float4* __restrict__ bterm, float k, float rho0,
-    float nu10, float eps, float3 grav, float dt, float4* __restrict__ acc,
+    const float4* __restrict__ vel, const float4* __restrict__ bterm, float k_r0, float rho0,
+    float nu10, float eps, float3 grav, float dt, Soa3 acc,
     float* __restrict__ x, float* __restrict__ y, float* __restrict__ z,
     float* __restrict__ vx, float* __restrict__ vy, float* __restrict__ vz, Tail tail)
 {
@@ -1109,17 +1130,15 @@ __global__ void __launch_bounds__(MB) k_sesph(uint32_t n, Fluid f,
     if (i < n) {
     const float4 me = f.pm[i];
     const float4 vi = vel[i];
-    const float pi = eos_sesph(vi.w, k, rho0);
-    const float pri = pi / (vi.w * vi.w);
+    const float pri = pressure_term_sesph(vi.w, k_r0, rho0);
     float ax = grav.x, ay = grav.y, az = grav.z;
     for_each_listed<R, 0, false, BATCH>(f, i, me,
         [&](uint32_t j, const float4& q, float dx, float dy, float dz, float l2) {
             const float4 vj = __ldg(vel + j);
-            const float pj = eos_sesph(vj.w, k, rho0);
             const float vdx = fmaf(vi.x - vj.x, dx, fmaf(vi.y - vj.y, dy, (vi.z - vj.z) * dz));
-            const float visc = (nu10 * q.w * vdx) / (vj.w * (l2 + eps));
-            const float prs = q.w * (pri + pj / (vj.w * vj.w));
-            const float s = (visc - prs) * pair_g<KIND>(f.kc, l2);
+            const float visc = (nu10 * vj.w * vdx) / (l2 + eps);
+            const float prs = pri + pressure_term_sesph(vj.w, k_r0, rho0);
+            const float s = q.w * (visc - prs) * pair_g<KIND>(f.kc, l2);
             ax += s * dx;
             ay += s * dy;
             az += s * dz;
@@ -1128,7 +1147,9 @@ __global__ void __launch_bounds__(MB) k_sesph(uint32_t n, Fluid f,
     ax -= pri * bt.x;
     ay -= pri * bt.y;
     az -= pri * bt.z;
-    acc[i] = make_float4(ax, ay, az, 0.f);
+    acc.x[i] = ax;
+    acc.y[i] = ay;
+    acc.z[i] = az;
     const float nvx = vi.x + dt * ax, nvy = vi.y + dt * ay, nvz = vi.z + dt * az;
     vn = store_state<BATCH>(tail, i, me.x + dt * nvx, me.y + dt * nvy, me.z + dt * nvz, nvx, nvy, nvz,
         x, y, z, vx, vy, vz);
@@ -1199,7 +1220,7 @@ __global__ void __launch_bounds__(MB) k_pcisph_predict_tiles(REYN_PCISPH_PREDICT
 // _write_pcisph_prs_acc (PCISPH.cu:21-56) + v += dt a in place
 #define REYN_PCISPH_PRESSURE_ARGS uint32_t n, Fluid f, const float* __restrict__ rho, \
     const float* __restrict__ pr, const float4* __restrict__ bterm, float k, float rho0, \
-    float r0i, float dt, float4* __restrict__ acc, float4* __restrict__ vel
+    float r0i, float dt, Soa3 acc, float4* __restrict__ vel
 #define REYN_PCISPH_PRESSURE_PASS n, f, rho, pr, bterm, k, rho0, r0i, dt, acc, vel
 
 template <int KIND, int R, bool BATCH>
@@ -1228,7 +1249,9 @@ __device__ __forceinline__ void pcisph_pressure(uint32_t i, REYN_PCISPH_PRESSURE
     ax = -ax - cb * bt.x;
     ay = -ay - cb * bt.y;
     az = -az - cb * bt.z;
-    acc[i] = make_float4(ax, ay, az, 0.f);
+    acc.x[i] = ax;
+    acc.y[i] = ay;
+    acc.z[i] = az;
     float4 v = vel[i];
     v.x += dt * ax;
     v.y += dt * ay;
@@ -1563,7 +1586,7 @@ void launch_iisph_pacc(unsigned nb, unsigned bs, cudaStream_t q, Tiles tl, bool 
     if constexpr (BATCH) {
         if (persist)
             k_iisph_pacc_tiles<KIND, R, MIX, MB><<<persistent_grid(
-                k_iisph_pacc_tiles<KIND, R, MIX, MB>, bs, nb), bs, 0, q>>>(a..., tl);
+                k_iisph_pacc_tiles<KIND, R, MIX, MB>, bs, tl.count), bs, 0, q>>>(a..., tl);
         else
             k_iisph_pacc<KIND, R, MIX, BATCH, MB><<<nb, bs, 0, q>>>(a...);
     } else if constexpr (occupancy_variant<KIND, MIX>) {
@@ -1580,7 +1603,7 @@ void launch_iisph_jacobi(unsigned nb, unsigned bs, cudaStream_t q, Tiles tl, boo
     if constexpr (BATCH) {
         if (persist)
             k_iisph_jacobi_tiles<KIND, R, MIX, MB><<<persistent_grid(
-                k_iisph_jacobi_tiles<KIND, R, MIX, MB>, bs, nb), bs, 0, q>>>(a..., tl);
+                k_iisph_jacobi_tiles<KIND, R, MIX, MB>, bs, tl.count), bs, 0, q>>>(a..., tl);
         else
             k_iisph_jacobi<KIND, R, MIX, BATCH, MB><<<nb, bs, 0, q>>>(a...);
     } else if constexpr (occupancy_variant<KIND, MIX>) {
@@ -1592,20 +1615,19 @@ void launch_iisph_jacobi(unsigned nb, unsigned bs, cudaStream_t q, Tiles tl, boo
 
 #define REYN_NONPRESSURE_ARGS uint32_t n, Fluid f, const float4* __restrict__ vel, \
     const uint2* __restrict__ velh, float nu10, float eps, float3 grav, float dt, \
-    float4* __restrict__ acc, float4* __restrict__ vel_out, uint2* __restrict__ velh_out, \
-    const float* __restrict__ p_old
+    float4* __restrict__ vel_out, uint2* __restrict__ velh_out, const float* __restrict__ p_old
 
 template <int KIND, int R, int MIX = 0, bool BATCH = false, int MB = NBR_THREADS>
 __global__ void __launch_bounds__(MB) k_nonpressure(REYN_NONPRESSURE_ARGS)
 {
-    nonpressure<KIND, R, MIX, BATCH>(n, f, vel, velh, nu10, eps, grav, dt, acc, vel_out,
+    nonpressure<KIND, R, MIX, BATCH>(n, f, vel, velh, nu10, eps, grav, dt, vel_out,
         velh_out, p_old);
 }
 
 template <int KIND, int R, int MIX, int MB>
 __global__ void __launch_bounds__(MB, (65536 / 48) / MB) k_nonpressure_occ(REYN_NONPRESSURE_ARGS)
 {
-    nonpressure<KIND, R, MIX, false>(n, f, vel, velh, nu10, eps, grav, dt, acc, vel_out,
+    nonpressure<KIND, R, MIX, false>(n, f, vel, velh, nu10, eps, grav, dt, vel_out,
         velh_out, p_old);
 }
 
@@ -1654,19 +1676,6 @@ __global__ void __launch_bounds__(MB) k_iisph_final(uint32_t n, Fluid f,
         x, y, z, vx, vy, vz);
     }
     tail_reduce(tail, vn);
-}
-
-// SESPH and PCISPH: the packed accelerations to the solver's SoA arrays
-__global__ void k_unpack_acc(uint32_t n, const float4* __restrict__ acc, float* __restrict__ ax,
-    float* __restrict__ ay, float* __restrict__ az)
-{
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n)
-        return;
-    const float4 a = acc[i];
-    ax[i] = a.x;
-    ay[i] = a.y;
-    az[i] = a.z;
 }
 
 __global__ void k_gather_p(uint32_t n, const uint32_t* __restrict__ perm,
@@ -1810,6 +1819,8 @@ void solver_step_t(reyn_solver& sv, reyn_particles& st, const Grid& grid,
     }
     const unsigned bs = P.block_size ? P.block_size : NBR_THREADS;
     const unsigned nb = blocks_for(n, bs);
+    const uint32_t shift = warp_shift(n);
+    const unsigned nbd = blocks_for(size_t(n) << (5 - shift), bs);
     const float rho0 = P.rho0;
     const float r0i = 1.f / (rho0 * rho0);
     const float nu10 = 10.f * P.nu;
@@ -1899,7 +1910,7 @@ void solver_step_t(reyn_solver& sv, reyn_particles& st, const Grid& grid,
     // over the tiles of the scenes still iterating
     Tiles tl {};
     if (ns)
-        tl = Tiles { grid.sid.get(), sv.scene_active.get(), n, nb };
+        tl = Tiles { grid.sid.get(), sv.scene_active.get(), n, blocks_for(n, bs) };
     const bool mixed = P.precision == REYN_PRECISION_MIXED;
     const bool rec16 = P.precision == REYN_PRECISION_MIXED_POS16;
     uint2* ACH = mixed ? sv.acch.get() : nullptr;
@@ -1908,6 +1919,7 @@ void solver_step_t(reyn_solver& sv, reyn_particles& st, const Grid& grid,
     uint4* REC0 = rec16 ? sv.rec0.get() : nullptr;
     uint4* REC1 = rec16 ? sv.rec1.get() : nullptr;
     f.acch = ACH;
+    const Soa3 ACC { sv.ax.get(), sv.ay.get(), sv.az.get() };
     // FP32 and MIXED: the pressure passes' records (x, y, z, m p) in place of
     // (x, y, z, m)
     Fluid fq = f;
@@ -1919,16 +1931,16 @@ void solver_step_t(reyn_solver& sv, reyn_particles& st, const Grid& grid,
         constexpr bool B = decltype(BC)::value;
         if (f.g.order == REYN_ORDER_XYZ)
             REYN_KERNEL("k_density", s,
-                k_density<K, R, true, MIX, B, MB><<<nb, bs, 0, s>>>(n, f, b, sv.rho.get(),
-                st.vel.get(), sv.bterm.get(), REC0, VH));
+                k_density<K, R, true, MIX, B, MB><<<nbd, bs, 0, s>>>(n, f, b, sv.rho.get(),
+                st.vel.get(), sv.bterm.get(), REC0, VH, sv.scheme == REYN_SESPH, shift));
         else
             REYN_KERNEL("k_density", s,
-                k_density<K, R, false, MIX, B, MB><<<nb, bs, 0, s>>>(n, f, b, sv.rho.get(),
-                st.vel.get(), sv.bterm.get(), REC0, VH));
+                k_density<K, R, false, MIX, B, MB><<<nbd, bs, 0, s>>>(n, f, b, sv.rho.get(),
+                st.vel.get(), sv.bterm.get(), REC0, VH, sv.scheme == REYN_SESPH, shift));
         if (sv.scheme == REYN_SESPH) {
             REYN_KERNEL("k_sesph", s,
                 k_sesph<K, R, B, MB><<<nb, bs, 0, s>>>(n, f, st.vel.get(), sv.bterm.get(),
-                P.k_sesph, rho0, nu10, eps, grav, dt, sv.acc.get(), X, Y, Z, VX, VY, VZ, tail));
+                P.k_sesph / rho0, rho0, nu10, eps, grav, dt, ACC, X, Y, Z, VX, VY, VZ, tail));
             iters = 1;
             if (gx) {
                 REYN_KERNEL("k_graph_single_pass", s,
@@ -1944,8 +1956,8 @@ void solver_step_t(reyn_solver& sv, reyn_particles& st, const Grid& grid,
             const float kp = (float)((sv.pcisph_delta / dt) / dt); // PCISPH.cu:65
             REYN_KERNEL("k_nonpressure", s,
                 launch_nonpressure<K, R, 0, B, MB>(nb, bs, s, n, f, (const float4*)st.vel.get(),
-                (const uint2*)nullptr, nu10, eps, grav, dt, sv.acc.get(), sv.vel2.get(),
-                (uint2*)nullptr, (const float*)nullptr));
+                (const uint2*)nullptr, nu10, eps, grav, dt, sv.vel2.get(), (uint2*)nullptr,
+                (const float*)nullptr));
             float4* v = sv.vel2.get();
             // one PCISPH iteration: prediction and pressure (a batch: over
             // the tiles of the scenes still iterating)
@@ -1953,19 +1965,19 @@ void solver_step_t(reyn_solver& sv, reyn_particles& st, const Grid& grid,
                 if (B && persist) {
                     REYN_KERNEL("k_pcisph_predict", q,
                         k_pcisph_predict_tiles<K, R, MB><<<persistent_grid(
-                        k_pcisph_predict_tiles<K, R, MB>, bs, nb), bs, 0, q>>>(n, f, v,
+                        k_pcisph_predict_tiles<K, R, MB>, bs, tl.count), bs, 0, q>>>(n, f, v,
                         sv.bterm.get(), dt, sv.rho.get(), kp, rho0, sv.p.get(), slot, tl));
                     REYN_KERNEL("k_pcisph_pressure", q,
                         k_pcisph_pressure_tiles<K, R, MB><<<persistent_grid(
-                        k_pcisph_pressure_tiles<K, R, MB>, bs, nb), bs, 0, q>>>(n, f, sv.rho.get(),
-                        sv.p.get(), sv.bterm.get(), kp, rho0, r0i, dt, sv.acc.get(), v, tl));
+                        k_pcisph_pressure_tiles<K, R, MB>, bs, tl.count), bs, 0, q>>>(n, f, sv.rho.get(),
+                        sv.p.get(), sv.bterm.get(), kp, rho0, r0i, dt, ACC, v, tl));
                 } else {
                     REYN_KERNEL("k_pcisph_predict", q,
                         k_pcisph_predict<K, R, B, MB><<<nb, bs, 0, q>>>(n, f, v, sv.bterm.get(),
                         dt, sv.rho.get(), kp, rho0, sv.p.get(), slot));
                     REYN_KERNEL("k_pcisph_pressure", q,
                         k_pcisph_pressure<K, R, B, MB><<<nb, bs, 0, q>>>(n, f, sv.rho.get(),
-                        sv.p.get(), sv.bterm.get(), kp, rho0, r0i, dt, sv.acc.get(), v));
+                        sv.p.get(), sv.bterm.get(), kp, rho0, r0i, dt, ACC, v));
                 }
             };
             if (gx) {
@@ -2032,7 +2044,7 @@ void solver_step_t(reyn_solver& sv, reyn_particles& st, const Grid& grid,
                 if (B && persist)
                     REYN_KERNEL("k_pacc_rec", q,
                         k_pacc_rec_tiles<K, R, MB><<<persistent_grid(
-                        k_pacc_rec_tiles<K, R, MB>, bs, nb), bs, 0, q>>>(n, f, rc,
+                        k_pacc_rec_tiles<K, R, MB>, bs, tl.count), bs, 0, q>>>(n, f, rc,
                         (const float4*)sv.gq.get(), r0i, RX, RY, gate, tl));
                 else
                     REYN_KERNEL("k_pacc_rec", q,
@@ -2043,7 +2055,7 @@ void solver_step_t(reyn_solver& sv, reyn_particles& st, const Grid& grid,
                 if (B && persist)
                     REYN_KERNEL("k_jacobi_rec", q,
                         k_jacobi_rec_tiles<K, R, MB><<<persistent_grid(
-                        k_jacobi_rec_tiles<K, R, MB>, bs, nb), bs, 0, q>>>(n, f, rc,
+                        k_jacobi_rec_tiles<K, R, MB>, bs, tl.count), bs, 0, q>>>(n, f, rc,
                         (const float4*)sv.gq.get(), (const float*)sv.sii.get(), sv.p.get(), dt,
                         P.omega, tiny, thr, slot, RY, RX, tl));
                 else
@@ -2116,11 +2128,11 @@ void solver_step_t(reyn_solver& sv, reyn_particles& st, const Grid& grid,
             REYN_KERNEL("k_final_rec", s,
                 k_final_rec<K, R, B, MB><<<nb, bs, 0, s>>>(n, f, rc,
                 (const float4*)sv.gq.get(), r0i, sv.vel2.get(), dt,
-                Soa3 { sv.ax.get(), sv.ay.get(), sv.az.get() }, RX, X, Y, Z, VX, VY, VZ, tail));
+                ACC, RX, X, Y, Z, VX, VY, VZ, tail));
         } else { // IISPH
             REYN_KERNEL("k_nonpressure", s,
                 launch_nonpressure<K, R, MIX, B, MB>(nb, bs, s, n, f, (const float4*)st.vel.get(),
-                (const uint2*)VH, nu10, eps, grav, dt, sv.acc.get(), sv.vel2.get(), VH2,
+                (const uint2*)VH, nu10, eps, grav, dt, sv.vel2.get(), VH2,
                 (const float*)sv.p.get()));
             const float tiny = tiny_threshold();
             auto pacc = [&] {
@@ -2204,7 +2216,7 @@ void solver_step_t(reyn_solver& sv, reyn_particles& st, const Grid& grid,
             }
             REYN_KERNEL("k_iisph_final", s,
                 k_iisph_final<K, R, MIX, B, MB><<<nb, bs, 0, s>>>(n, fq, sv.p.get(), sv.gq.get(),
-                r0i, sv.vel2.get(), dt, Soa3 { sv.ax.get(), sv.ay.get(), sv.az.get() }, X, Y, Z,
+                r0i, sv.vel2.get(), dt, ACC, X, Y, Z,
                 VX, VY, VZ, tail));
         }
     };
@@ -2225,11 +2237,6 @@ void solver_step_t(reyn_solver& sv, reyn_particles& st, const Grid& grid,
         else
             body(KC, RC, std::integral_constant<int, 0> {}, std::false_type {});
     });
-    if (sv.scheme != REYN_IISPH) {
-        REYN_KERNEL("k_unpack_acc", s,
-            k_unpack_acc<<<blocks_for(n, THREADS), THREADS, 0, s>>>(n, sv.acc.get(), sv.ax.get(),
-            sv.ay.get(), sv.az.get()));
-    }
     st.packed_valid = false; // positions moved: the packed copy is stale
     st.version += 1;
     if (prekeyed) {

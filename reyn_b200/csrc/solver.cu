@@ -65,7 +65,6 @@ void ensure_buffers(reyn_solver& sv, uint32_t n)
     sv.ax.resize(n);
     sv.ay.resize(n);
     sv.az.resize(n);
-    sv.acc.resize(n);
     sv.vel2.resize(n);
     sv.bterm.resize(n);
     sv.nbr.resize(list_capacity(n));
@@ -80,8 +79,10 @@ void ensure_buffers(reyn_solver& sv, uint32_t n)
     }
     if (sv.scheme == REYN_IISPH) {
         sv.gq.resize(n);
-        if (sv.prm.precision != REYN_PRECISION_MIXED_POS16)
+        if (sv.prm.precision != REYN_PRECISION_MIXED_POS16) {
+            sv.acc.resize(n);
             sv.xq.resize(n);
+        }
     }
     if (sv.p.size() != n) {
         sv.p.resize(n);
