@@ -8,9 +8,11 @@
 #include <cstdint>
 #include <cstring>
 #include <exception>
+#include <functional>
 #include <new>
 #include <string>
 #include <utility>
+#include <vector>
 
 #include "reyn_b200.h"
 
@@ -90,8 +92,8 @@ inline void require(bool ok, const char* msg)
         fail(REYN_ERR_INVALID, msg);
 }
 
-// Owning device allocation of `n` elements of T (cudaMalloc'ed once, resized
-// only when a larger size is requested).
+// Device allocation of `n` elements of T (cudaMalloc'ed once, resized only when
+// a larger size is requested), or a part of a Slab, which then owns the memory.
 template <class T> class DevArray {
 public:
     DevArray() = default;
@@ -103,6 +105,7 @@ public:
         : p_(std::exchange(o.p_, nullptr))
         , n_(std::exchange(o.n_, 0))
         , cap_(std::exchange(o.cap_, 0))
+        , part_(std::exchange(o.part_, false))
     {
     }
     DevArray& operator=(DevArray&& o) noexcept
@@ -112,6 +115,7 @@ public:
             p_ = std::exchange(o.p_, nullptr);
             n_ = std::exchange(o.n_, 0);
             cap_ = std::exchange(o.cap_, 0);
+            part_ = std::exchange(o.part_, false);
         }
         return *this;
     }
@@ -126,6 +130,14 @@ public:
         }
         n_ = n;
     }
+    // becomes n elements at p, inside memory that a Slab owns
+    void adopt(T* p, size_t n)
+    {
+        release();
+        p_ = p;
+        n_ = cap_ = n;
+        part_ = true;
+    }
     void zero(cudaStream_t s)
     {
         if (n_)
@@ -138,19 +150,49 @@ public:
         std::swap(p_, o.p_);
         std::swap(n_, o.n_);
         std::swap(cap_, o.cap_);
+        std::swap(part_, o.part_);
     }
 
 private:
     void release() noexcept
     {
-        if (p_)
+        if (p_ && !part_)
             cudaFree(p_);
         p_ = nullptr;
         n_ = cap_ = 0;
+        part_ = false;
     }
     T* p_ = nullptr;
     size_t n_ = 0;
     size_t cap_ = 0;
+    bool part_ = false;
+};
+
+// One device allocation for several DevArrays: add() each with its size, then
+// allocate(). An allocation and its release cost the host far more than what
+// short-lived or small arrays are used for.
+class Slab {
+public:
+    template <class T> void add(DevArray<T>& a, size_t n)
+    {
+        const size_t at = bytes_;
+        bytes_ += (n * sizeof(T) + 255) / 256 * 256;
+        parts_.push_back([&a, n, at](unsigned char* base) {
+            a.adopt(reinterpret_cast<T*>(base + at), n);
+        });
+    }
+    void allocate()
+    {
+        mem_.resize(bytes_);
+        for (auto& part : parts_)
+            part(mem_.get());
+        parts_.clear();
+    }
+
+private:
+    DevArray<unsigned char> mem_;
+    size_t bytes_ = 0;
+    std::vector<std::function<void(unsigned char*)>> parts_;
 };
 
 // Pinned host scratch for small device->host readbacks.

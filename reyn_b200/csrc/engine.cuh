@@ -149,6 +149,7 @@ struct reyn_boundary {
     uint32_t nb = 0;
     float h = 0.f;
     float lo[3] = { 0.f, 0.f, 0.f }, hi[3] = { 0.f, 0.f, 0.f }; // the samples' bounds
+    reyn::Slab points, cells; // the memory of the arrays below and the grid's
     reyn::Grid grid;
     reyn::DevArray<float> x, y, z, m;
     reyn::DevArray<float4> pm;

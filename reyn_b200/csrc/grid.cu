@@ -366,11 +366,14 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply(
         out[C] = offset + total;
 }
 
+// the partial sums exclusive_scan needs for C counts
+static size_t scan_parts(size_t C) { return (C + SCAN_TILE - 1) / SCAN_TILE + 1; }
+
 void exclusive_scan(const uint32_t* in, int64_t C, DevArray<uint32_t>& part,
     uint32_t* out, cudaStream_t s, uint32_t* fold_status)
 {
     const uint32_t nparts = (uint32_t)((C + SCAN_TILE - 1) / SCAN_TILE);
-    part.resize(size_t(nparts) + 1);
+    part.resize(scan_parts(size_t(C)));
     REYN_KERNEL("k_scan_tiles", s,
         k_scan_tiles<<<nparts, SCAN_THREADS, 0, s>>>(in, C, part.get(), fold_status));
     REYN_KERNEL("k_scan_apply", s,
@@ -840,26 +843,53 @@ inline float from_ordered_bits(unsigned u)
     return f;
 }
 
-// bounding box of the samples (sample_boundary.cu:415-416: xs.min() ...)
-__global__ void k_bounds(uint32_t n, const float* __restrict__ x, const float* __restrict__ y,
-    const float* __restrict__ z, unsigned* __restrict__ box)
+// bounding box of each scene's samples (sample_boundary.cu:415-416: xs.min()
+// ...; one scene: all of them, first == nullptr): six ordered words a scene,
+// minima then complemented maxima, so that one initial value (all ones) and
+// one atomic serve both. blockIdx.y is the scene, whose samples its blocks
+// share; a block reduces first (an atomic a sample serialises on the six
+// words: 59 us over 400k samples against 13).
+__global__ void __launch_bounds__(THREADS) k_bounds(uint32_t n,
+    const uint32_t* __restrict__ first, const float* __restrict__ x,
+    const float* __restrict__ y, const float* __restrict__ z, unsigned* __restrict__ box)
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n)
-        return;
-    const float v[3] = { x[i], y[i], z[i] };
+    const uint32_t sc = blockIdx.y;
+    const uint32_t end = first ? first[sc + 1] : n;
+    unsigned v[6];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        atomicMin(box + a, ordered_bits(v[a]));
-        atomicMax(box + 3 + a, ordered_bits(v[a]));
+    for (int a = 0; a < 6; ++a)
+        v[a] = 0xffffffffu;
+    for (uint32_t i = (first ? first[sc] : 0u) + blockIdx.x * THREADS + threadIdx.x; i < end;
+         i += gridDim.x * THREADS) {
+        const unsigned b[3] = { ordered_bits(x[i]), ordered_bits(y[i]), ordered_bits(z[i]) };
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            v[a] = min(v[a], b[a]);
+            v[3 + a] = min(v[3 + a], ~b[a]);
+        }
     }
+    __shared__ unsigned part[6];
+    if (threadIdx.x < 6)
+        part[threadIdx.x] = 0xffffffffu;
+    __syncthreads();
+#pragma unroll
+    for (int a = 0; a < 6; ++a) {
+        const unsigned w = __reduce_min_sync(0xffffffffu, v[a]);
+        if ((threadIdx.x & 31) == 0)
+            atomicMin(part + a, w);
+    }
+    __syncthreads();
+    if (threadIdx.x < 6)
+        atomicMin(box + 6 * sc + threadIdx.x, part[threadIdx.x]);
 }
 
 // one Akinci mass refinement (sample_boundary.cu:250-265), double-buffered:
-// m_i <- rho0 m_i / sum_j m_j W_B3(x_ij), support 2h
+// m_i <- rho0 m_i / sum_j m_j W_B3(x_ij), support 2h; the last one also writes
+// the masses alone
 template <int R>
 __global__ void __launch_bounds__(NBR_THREADS) k_boundary_mass(uint32_t n, GridView g,
-    KernelConst kc, const float4* __restrict__ pts, float rho0, float4* __restrict__ out)
+    KernelConst kc, const float4* __restrict__ pts, float rho0, float4* __restrict__ out,
+    float* __restrict__ m_out)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
@@ -872,33 +902,58 @@ __global__ void __launch_bounds__(NBR_THREADS) k_boundary_mass(uint32_t n, GridV
         [&](uint32_t, const float4& q, float, float, float, float l2) {
             sum += q.w * pair_w<K_B3>(kc, l2);
         });
-    out[i] = make_float4(me.x, me.y, me.z, rho0 * me.w / sum);
+    const float m = rho0 * me.w / sum;
+    out[i] = make_float4(me.x, me.y, me.z, m);
+    if (m_out)
+        m_out[i] = m;
 }
 
-// marks the (2R+1)^3 cells around every boundary sample
+// marks the (2R+1)^2 cells of every boundary sample's own x around it; the
+// runs along x come from k_widen_near. (Marking all 125 cells per sample takes
+// 99 us over 400k samples, mostly stores to cells already marked; the two
+// kernels take 38.)
 __global__ void k_mark_near(uint32_t n, GridView g, const float4* __restrict__ pts,
-    uint8_t* __restrict__ near)
+    uint8_t* __restrict__ mark)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
         return;
     const float4 me = pts[i];
     g = at_scene(g, scene_of(g, i)); // batched: the sample's own scene grid
-    near += g.key_base;
+    mark += g.key_base;
     const int3 c = clamp_cell(g, cell_of(g, me.x, me.y, me.z), 2);
     for (int dz = -2; dz <= 2; ++dz)
-        for (int dy = -2; dy <= 2; ++dy) {
-            const int base = (c.z + dz) * g.nxny + (c.y + dy) * g.nx + c.x;
-            for (int dx = -2; dx <= 2; ++dx)
-                near[base + dx] = 1;
-        }
+        for (int dy = -2; dy <= 2; ++dy)
+            mark[(c.z + dz) * g.nxny + (c.y + dy) * g.nx + c.x] = 1;
 }
 
-__global__ void k_unpack_mass(uint32_t n, const float4* __restrict__ pts, float* __restrict__ m)
+// near[c] = any of mark[c - 2 .. c + 2], sixteen cells a thread. Marked cells
+// lie at least two cells inside their row, so no mark reaches another row. Both
+// arrays are padded to sixteen bytes.
+__global__ void k_widen_near(size_t words, const uint32_t* __restrict__ mark,
+    uint32_t* __restrict__ near)
+{
+    const size_t t = (size_t(blockIdx.x) * blockDim.x + threadIdx.x) * 4;
+    if (t >= words)
+        return;
+    const uint4 v = *reinterpret_cast<const uint4*>(mark + t);
+    const uint32_t w[6] = { t ? mark[t - 1] : 0u, v.x, v.y, v.z, v.w,
+        t + 4 < words ? mark[t + 4] : 0u };
+    uint32_t o[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const uint32_t p = w[k], q = w[k + 1], r = w[k + 2];
+        o[k] = q | __funnelshift_l(p, q, 8) | __funnelshift_l(p, q, 16)
+            | __funnelshift_r(q, r, 8) | __funnelshift_r(q, r, 16);
+    }
+    *reinterpret_cast<uint4*>(near + t) = make_uint4(o[0], o[1], o[2], o[3]);
+}
+
+__global__ void k_fill(uint32_t n, float v, float* __restrict__ out)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n)
-        m[i] = pts[i].w;
+        out[i] = v;
 }
 
 void boundary_build(reyn_boundary& b, const float* bx, const float* by, const float* bz,
@@ -912,102 +967,111 @@ void boundary_build(reyn_boundary& b, const float* bx, const float* by, const fl
         return;
     require(bx && by && bz, "null boundary positions");
     require(bm || mass_iters > 0, "at least one mass refinement iteration is required");
-    DevArray<unsigned> box(6);
-    const unsigned init[6] = { 0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u };
-    REYN_CUDA(cudaMemcpyAsync(box.get(), init, sizeof(init), cudaMemcpyHostToDevice, s));
+    // what the samples need, in one allocation; what the cells need follows
+    // once their number is known
+    require(n_scenes <= 65535, "1 .. 65535 scenes");
+    const uint32_t ns = std::max(1u, n_scenes);
+    DevArray<unsigned> box;
+    DevArray<uint32_t> sfirst;
+    DevArray<float4> other;
+    b.points.add(box, size_t(6) * ns);
+    b.points.add(sfirst, n_scenes ? n_scenes + 1 : 0);
+    b.points.add(other, bm ? 0 : nb);
+    b.points.add(b.pm, nb);
+    for (DevArray<float>* a : { &b.x, &b.y, &b.z, &b.m })
+        b.points.add(*a, nb);
+    for (DevArray<uint32_t>* a : { &b.grid.keys, &b.grid.slots, &b.grid.sorted, &b.grid.split })
+        b.points.add(*a, nb);
+    b.points.add(b.grid.status, 3);
+    b.points.allocate();
+    REYN_CUDA(cudaMemsetAsync(box.get(), 0xff, box.size() * sizeof(unsigned), s));
+    if (n_scenes) {
+        for (uint32_t k = 0; k < n_scenes; ++k)
+            require(scene_first[k + 1] > scene_first[k],
+                "every scene of a batched boundary needs samples");
+        REYN_CUDA(cudaMemcpyAsync(sfirst.get(), scene_first, (n_scenes + 1) * sizeof(uint32_t),
+            cudaMemcpyHostToDevice, s));
+    }
+    const dim3 bgrid(std::min(blocks_for(nb / ns + 1, THREADS * 4), 148u * 4u), ns);
     REYN_KERNEL("k_bounds", s,
-        k_bounds<<<blocks_for(nb, THREADS), THREADS, 0, s>>>(nb, bx, by, bz, box.get()));
-    unsigned hb[6];
-    REYN_CUDA(cudaMemcpyAsync(hb, box.get(), sizeof(hb), cudaMemcpyDeviceToHost, s));
+        k_bounds<<<bgrid, THREADS, 0, s>>>(nb, n_scenes ? sfirst.get() : nullptr, bx, by, bz,
+        box.get()));
+    std::vector<unsigned> hb(box.size());
+    REYN_CUDA(cudaMemcpyAsync(hb.data(), box.get(), hb.size() * sizeof(unsigned),
+        cudaMemcpyDeviceToHost, s));
     REYN_CUDA(cudaStreamSynchronize(s));
-    float lo[3], hi[3];
+    std::vector<float> los(size_t(3) * ns), his(size_t(3) * ns);
+    unsigned all[6] = { ~0u, ~0u, ~0u, ~0u, ~0u, ~0u };
+    for (uint32_t k = 0; k < ns; ++k)
+        for (int a = 0; a < 3; ++a) {
+            los[3 * k + a] = from_ordered_bits(hb[6 * k + a]);
+            his[3 * k + a] = from_ordered_bits(~hb[6 * k + 3 + a]);
+            all[a] = std::min(all[a], hb[6 * k + a]);
+            all[3 + a] = std::min(all[3 + a], hb[6 * k + 3 + a]);
+        }
     for (int a = 0; a < 3; ++a) {
-        lo[a] = from_ordered_bits(hb[a]);
-        hi[a] = from_ordered_bits(hb[3 + a]);
-        b.lo[a] = lo[a];
-        b.hi[a] = hi[a];
+        b.lo[a] = from_ordered_bits(all[a]);
+        b.hi[a] = from_ordered_bits(~all[3 + a]);
     }
     // the boundary grid: support 2h over the samples' own bounds, reference
     // geometry (sample_boundary.cu:420-428)
-    b.grid.geom = make_geom(lo, hi, 2.f * h, 0.5f);
+    b.grid.geom = make_geom(b.lo, b.hi, 2.f * h, 0.5f);
     if (n_scenes) {
         // batched: every scene's samples get the grid a boundary of their
         // own would get (over their own bounds), keyed scene after scene
-        DevArray<unsigned> sbox(size_t(6) * n_scenes);
-        std::vector<unsigned> sinit(size_t(6) * n_scenes);
-        for (uint32_t k = 0; k < n_scenes; ++k)
-            std::copy(init, init + 6, sinit.begin() + 6 * size_t(k));
-        REYN_CUDA(cudaMemcpyAsync(sbox.get(), sinit.data(), sinit.size() * sizeof(unsigned),
-            cudaMemcpyHostToDevice, s));
-        for (uint32_t k = 0; k < n_scenes; ++k) {
-            const uint32_t a = scene_first[k], cnt = scene_first[k + 1] - a;
-            require(cnt > 0, "every scene of a batched boundary needs samples");
-            REYN_KERNEL("k_bounds", s,
-                k_bounds<<<blocks_for(cnt, THREADS), THREADS, 0, s>>>(cnt, bx + a, by + a, bz + a,
-                sbox.get() + 6 * size_t(k)));
-        }
-        std::vector<unsigned> hsb(sinit.size());
-        REYN_CUDA(cudaMemcpyAsync(hsb.data(), sbox.get(), hsb.size() * sizeof(unsigned),
-            cudaMemcpyDeviceToHost, s));
-        REYN_CUDA(cudaStreamSynchronize(s));
         std::vector<GridGeom> geoms(n_scenes);
-        for (uint32_t k = 0; k < n_scenes; ++k) {
-            float slo[3], shi[3];
-            for (int a = 0; a < 3; ++a) {
-                slo[a] = from_ordered_bits(hsb[6 * k + a]);
-                shi[a] = from_ordered_bits(hsb[6 * k + 3 + a]);
-            }
-            geoms[k] = make_geom(slo, shi, 2.f * h, 0.5f);
-        }
+        for (uint32_t k = 0; k < n_scenes; ++k)
+            geoms[k] = make_geom(&los[3 * size_t(k)], &his[3 * size_t(k)], 2.f * h, 0.5f);
         b.grid.set_scenes(scene_first, n_scenes, geoms.data(), s);
     }
+    const size_t C = size_t(b.grid.total_keys());
+    b.cells.add(b.grid.counts, C);
+    b.cells.add(b.grid.prefix, C + 1);
+    b.cells.add(b.grid.scan_part, scan_parts(C));
+    b.cells.add(b.near, C);
+    b.cells.allocate();
+    b.grid.counts_dirty = true; // not yet zero
     b.grid.build(bx, by, bz, nb, s);
     b.grid.check_status(s, "boundary grid");
-    b.x.resize(nb);
-    b.y.resize(nb);
-    b.z.resize(nb);
-    b.m.resize(nb);
-    b.pm.resize(nb);
-    DevArray<float> ones;
-    if (!bm) {
-        ones.resize(nb);
-        std::vector<float> h1(nb, 1.f); // m_0 = 1 (sample_boundary.cu:277)
-        REYN_CUDA(cudaMemcpyAsync(ones.get(), h1.data(), nb * sizeof(float),
-            cudaMemcpyHostToDevice, s));
-        REYN_CUDA(cudaStreamSynchronize(s));
-    }
     GatherArgs a {};
-    a.count = 4;
+    a.count = bm ? 4 : 3;
     a.src[0] = bx;
     a.src[1] = by;
     a.src[2] = bz;
-    a.src[3] = bm ? bm : ones.get();
+    a.src[3] = bm;
     a.dst[0] = b.x.get();
     a.dst[1] = b.y.get();
     a.dst[2] = b.z.get();
     a.dst[3] = b.m.get();
     launch_gather(nb, b.grid.sorted.get(), a, s);
+    if (!bm) // m_0 = 1 (sample_boundary.cu:277)
+        REYN_KERNEL("k_fill", s,
+            k_fill<<<blocks_for(nb, THREADS), THREADS, 0, s>>>(nb, 1.f, b.m.get()));
     REYN_KERNEL("k_pack_positions", s,
         k_pack_positions<<<blocks_for(nb, THREADS), THREADS, 0, s>>>(
         nb, nullptr, b.x.get(), b.y.get(), b.z.get(), b.m.get(), b.pm.get()));
     b.grid.reordered = true;
-    b.near.resize(size_t(b.grid.total_keys()));
-    b.near.zero(s);
+    // the marks take the place of the cell counts, which the scatter left at
+    // zero (one byte a cell; the array is four times as long)
+    uint32_t* mark = b.grid.counts.get();
+    b.grid.counts_dirty = true;
     REYN_KERNEL("k_mark_near", s,
         k_mark_near<<<blocks_for(nb, THREADS), THREADS, 0, s>>>(nb, b.view(), b.pm.get(),
-            b.near.get()));
+            reinterpret_cast<uint8_t*>(mark)));
+    const size_t words = (C + 15) / 16 * 4;
+    REYN_KERNEL("k_widen_near", s,
+        k_widen_near<<<blocks_for(words / 4, THREADS), THREADS, 0, s>>>(words, mark,
+            reinterpret_cast<uint32_t*>(b.near.get())));
     if (!bm) {
-        DevArray<float4> other(nb);
         const GridView v = b.view();
         const KernelConst kc = make_kernel(K_B3, 2.f * h);
         for (uint32_t it = 0; it < mass_iters; ++it) {
             REYN_KERNEL("k_boundary_mass", s,
                 k_boundary_mass<2><<<blocks_for(nb, NBR_THREADS), NBR_THREADS, 0, s>>>(
-                nb, v, kc, b.pm.get(), rho0, other.get()));
+                nb, v, kc, b.pm.get(), rho0, other.get(),
+                it + 1 == mass_iters ? b.m.get() : nullptr));
             b.pm.swap(other);
         }
-        REYN_KERNEL("k_unpack_mass", s,
-            k_unpack_mass<<<blocks_for(nb, THREADS), THREADS, 0, s>>>(nb, b.pm.get(), b.m.get()));
         REYN_CUDA(cudaStreamSynchronize(s));
     }
 }
