@@ -77,11 +77,11 @@ struct Grid {
     DevArray<uint32_t> counts; // C, all zero between builds
     DevArray<uint32_t> prefix; // C + 1
     DevArray<uint32_t> keys;   // n
-    DevArray<uint32_t> slots;  // n, unordered counting-sort output
+    DevArray<uint32_t> slots;  // n, counting-sort output
     DevArray<uint32_t> sorted; // n, canonical order (the permutation)
-    DevArray<uint32_t> split;  // n, particles of cells split across warps
+    DevArray<uint8_t> split;   // n, marks slots of cells split across warps
     DevArray<uint32_t> scan_part;
-    DevArray<uint32_t> status; // StatusBits, the split-cell particle count, pre-key StatusBits
+    DevArray<uint32_t> status; // StatusBits, pre-key StatusBits
     DevArray<float> extra_tmp; // reorder staging of caller arrays
     mutable DevArray<float4> pts_tmp; // packed positions for statistics
     uint32_t n = 0;
@@ -101,12 +101,14 @@ struct Grid {
     void set_scenes(const uint32_t* first, uint32_t n_scenes, const GridGeom* geoms,
         cudaStream_t s);
     bool counts_dirty = false; // a build stopped between histogram and scatter
+    bool split_dirty = false;  // split may hold marks
+    bool unresolved = false;   // sorted still to be formed from slots (resolve)
     bool reordered = false;    // last build was construct_and_reorder
     const reyn_particles* reordered_state = nullptr;
     uint64_t reorder_epoch = 0; // state epoch produced by that reorder
     const float* built_pos[3] = { nullptr, nullptr, nullptr }; // positions of the last build
     // Keys and histogram of the next build, computed by the integrating
-    // kernel of a solver step on this grid's reordered state (status word 2
+    // kernel of a solver step on this grid's reordered state (status word 1
     // holds that kernel's status bits): valid while the state is unchanged
     // since (same arrays and version).
     bool prekey_pending = false;
@@ -119,9 +121,12 @@ struct Grid {
     // counting-sort build over positions: keys, counts, prefix, canonical
     // `sorted`; flags particles outside the grid in `status`. With `st` (the
     // state whose current positions x, y, z are) a pending pre-keyed
-    // histogram of that state is used instead of computing the keys.
+    // histogram of that state is used instead of computing the keys. With
+    // reorder_follows `sorted` is left to reorder_state's gather.
     void build(const float* x, const float* y, const float* z, uint32_t n,
-        cudaStream_t s, const reyn_particles* st = nullptr);
+        cudaStream_t s, const reyn_particles* st = nullptr, bool reorder_follows = false);
+    // forms `sorted` if a build left it
+    void resolve(cudaStream_t s);
     // drops a pending pre-keyed histogram (its counts are cleared)
     void drop_prekey(cudaStream_t s);
     // host check of the status word (synchronises)

@@ -111,6 +111,8 @@ struct HostState {
         g.n = grid_n;
         g.reordered = reordered;
         g.counts_dirty = counts_dirty;
+        g.split_dirty = false;
+        g.unresolved = false;
         g.reordered_state = reordered_state;
         g.reorder_epoch = reorder_epoch;
         sv.p_state = p_state;
@@ -147,7 +149,7 @@ void capture(reyn_step_graph& gr, int k)
     profile_record(&gr.ctx.top_names);
     try {
         REYN_CUDA(cudaMemsetAsync(gr.stats.get(), 0, sizeof(GraphStats), s));
-        g.build(st.cur[FX].get(), st.cur[FY].get(), st.cur[FZ].get(), st.n, s);
+        g.build(st.cur[FX].get(), st.cur[FY].get(), st.cur[FZ].get(), st.n, s, nullptr, true);
         reorder_state(st, g, nullptr, 0, s);
         solver_step(sv, st, g, gr.bdy, gr.dt, s, gr.bounded ? gr.lo : nullptr,
             gr.bounded ? gr.hi : nullptr);

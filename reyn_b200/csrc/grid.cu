@@ -1,8 +1,8 @@
 // Uniform-grid build on the B200: cell keys + warp-aggregated histogram,
-// tiled prefix scan over all cells, counting-sort scatter, a canonicalising
-// pass that makes the order inside each cell ascending (deterministic), and
-// one fused gather that permutes every particle array and writes the packed
-// (x, y, z, m) / (v, rho) copies the neighbour loops read.
+// tiled prefix scan over all cells, counting-sort scatter, and one fused gather
+// that settles the order inside each cell (ascending, deterministic), permutes
+// every particle array and writes the packed (x, y, z, m) / (v, rho) copies the
+// neighbour loops read.
 //
 // Reference: UniformGridBuilder (uniformgrid.cu:20-181, uniformgrid.cuh:
 // 200-489). The reference's scatter slot comes from atomicSub and is
@@ -151,21 +151,18 @@ __global__ void k_canonical(uint32_t n, const uint32_t* __restrict__ slots,
     sorted[st + rank] = p;
 }
 
-// counting-sort scatter straight into the canonical order (uniformgrid.cu:
-// 40-63, with the order inside a cell made deterministic: ascending index).
-// A warp's lanes hold consecutive indices, so a cell whose particles all lie
-// in one warp (its count, prefix[key + 1] - prefix[key], equals the number of
-// lanes holding its key) is placed by lane rank; the leader returns the
-// cell's counter to zero. A cell split across warps takes counting-sort
-// slots (atomicSub, which also returns its counter to zero) into `slots`,
-// and its particles are listed in `split` (count in *nsplit) for
-// k_rank_split. In a state reordered by the previous step's grid nearly
-// every cell is whole. Blocks of THREADS threads.
+// counting-sort scatter, in canonical order (ascending index inside a cell)
+// where a warp can tell (uniformgrid.cu:40-63, whose order inside a cell is
+// nondeterministic). A warp's lanes hold consecutive indices, so a cell whose
+// particles all lie in one warp (its count, prefix[key + 1] - prefix[key],
+// equals the number of lanes holding its key) is placed by lane rank; the
+// leader returns the cell's counter to zero. A cell split across warps takes
+// counting-sort slots (atomicSub, which also returns its counter to zero),
+// marked in `split` for whoever reads the slots next (canonical_slot). In a
+// state reordered by the previous step's grid nearly every cell is whole.
 __global__ void __launch_bounds__(THREADS) k_scatter_stable(uint32_t n,
-    const uint32_t* __restrict__ keys,
-    const uint32_t* __restrict__ prefix, uint32_t* __restrict__ counts,
-    uint32_t* __restrict__ slots, uint32_t* __restrict__ sorted, uint32_t* __restrict__ split,
-    uint32_t* __restrict__ nsplit)
+    const uint32_t* __restrict__ keys, const uint32_t* __restrict__ prefix,
+    uint32_t* __restrict__ counts, uint32_t* __restrict__ slots, uint8_t* __restrict__ split)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = i < n;
@@ -189,57 +186,49 @@ __global__ void __launch_bounds__(THREADS) k_scatter_stable(uint32_t n,
             top = atomicSub(counts + key, g);
     }
     top = __shfl_sync(0xffffffffu, top, leader);
-    if (valid) {
-        if (whole)
-            sorted[st + rank] = i;
-        else
-            slots[st + top - g + rank] = i;
+    if (!valid)
+        return;
+    if (whole) {
+        slots[st + rank] = i;
+    } else {
+        const uint32_t t = st + top - g + rank;
+        slots[t] = i;
+        split[t] = 1;
     }
-    // the split list: one atomic per block that has split cells (after a
-    // developed flow's step a few percent of the particles land in cells
-    // whose other particles sit in another warp; an atomic per warp then
-    // serialises on the one counter)
-    if (!__syncthreads_or(valid && !whole))
-        return; // the block holds no particle of a split cell
-    const unsigned sm = __ballot_sync(0xffffffffu, valid && !whole);
-    __shared__ uint32_t warp_base[THREADS / 32];
-    __shared__ uint32_t block_base;
-    const int w = threadIdx.x >> 5;
-    if (lane == 0)
-        warp_base[w] = __popc(sm);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t tot = 0;
-        for (int k = 0; k < int(blockDim.x >> 5); ++k) {
-            const uint32_t c = warp_base[k];
-            warp_base[k] = tot;
-            tot += c;
-        }
-        block_base = atomicAdd(nsplit, tot);
-    }
-    __syncthreads();
-    if (valid && !whole)
-        split[block_base + warp_base[w] + __popc(sm & ((1u << lane) - 1u))] = i;
 }
 
-// the canonical place of each particle of a split cell: its cell's start plus
-// the number of smaller indices among the cell's slots (grid-stride over the
-// split list, whose length is known on the device only)
-__global__ void k_rank_split(const uint32_t* __restrict__ nsplit,
-    const uint32_t* __restrict__ split, const uint32_t* __restrict__ slots,
-    const uint32_t* __restrict__ keys, const uint32_t* __restrict__ prefix,
-    uint32_t* __restrict__ sorted)
+// Where a slot's particle p belongs: the slot itself, or, in a cell split
+// across warps, the cell's start plus the number of smaller indices among the
+// cell's slots. Clears the slot's mark (split is all zero between builds).
+struct SplitCells {
+    const uint32_t* __restrict__ slots;
+    uint8_t* __restrict__ split;
+    const uint32_t* __restrict__ keys;
+    const uint32_t* __restrict__ prefix;
+    uint32_t* __restrict__ sorted;
+};
+
+__device__ __forceinline__ uint32_t canonical_slot(const SplitCells& c, uint32_t s, uint32_t p)
 {
-    const uint32_t m = *nsplit;
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < m; t += gridDim.x * blockDim.x) {
-        const uint32_t p = split[t];
-        const uint32_t key = keys[p];
-        const uint32_t st = prefix[key], en = prefix[key + 1];
-        uint32_t rank = 0;
-        for (uint32_t q = st; q < en; ++q)
-            rank += (slots[q] < p) ? 1u : 0u;
-        sorted[st + rank] = p;
-    }
+    if (!c.split[s])
+        return s;
+    c.split[s] = 0;
+    const uint32_t key = c.keys[p];
+    const uint32_t st = c.prefix[key], en = c.prefix[key + 1];
+    uint32_t rank = 0;
+    for (uint32_t q = st; q < en; ++q)
+        rank += (c.slots[q] < p) ? 1u : 0u;
+    return st + rank;
+}
+
+// the canonical order alone, for builds without a reorder
+__global__ void __launch_bounds__(THREADS) k_resolve(uint32_t n, SplitCells c)
+{
+    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= n)
+        return;
+    const uint32_t p = c.slots[s];
+    c.sorted[canonical_slot(c, s, p)] = p;
 }
 
 // ---- exclusive scan over all cells ----------------------------------------
@@ -307,10 +296,10 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_tiles(
     const uint32_t* __restrict__ in, int64_t C, uint32_t* __restrict__ part,
     uint32_t* __restrict__ fold_status)
 {
-    // a pre-keyed build: the keys' status bits (word 2) become the build's
+    // a pre-keyed build: the keys' status bits (word 1) become the build's
     if (fold_status && blockIdx.x == 0 && threadIdx.x == 0) {
-        fold_status[0] = fold_status[2];
-        fold_status[2] = 0u;
+        fold_status[0] = fold_status[1];
+        fold_status[1] = 0u;
     }
     const int64_t base = int64_t(blockIdx.x) * SCAN_TILE + int64_t(threadIdx.x) * SCAN_PER_THREAD;
     uint32_t v[SCAN_PER_THREAD];
@@ -388,8 +377,17 @@ void Grid::drop_prekey(cudaStream_t s)
     }
 }
 
+void Grid::resolve(cudaStream_t s)
+{
+    if (unresolved && n)
+        REYN_KERNEL("k_resolve", s,
+            k_resolve<<<blocks_for(n, THREADS), THREADS, 0, s>>>(n,
+            SplitCells { slots.get(), split.get(), keys.get(), prefix.get(), sorted.get() }));
+    unresolved = false;
+}
+
 void Grid::build(const float* x, const float* y, const float* z, uint32_t np,
-    cudaStream_t s, const reyn_particles* st)
+    cudaStream_t s, const reyn_particles* st, bool reorder_follows)
 {
     const int64_t C = total_keys();
     require(!n_scenes || np == first[n_scenes], "particle count differs from the scenes' total");
@@ -407,16 +405,21 @@ void Grid::build(const float* x, const float* y, const float* z, uint32_t np,
         prefix.resize(size_t(C) + 1);
         counts_dirty = false;
     }
-    if (status.size() < 3)
-        status.resize(3);
-    // the status bits and the split-cell count (a pre-keyed build keeps word
-    // 2, the keys' status, which the scan folds into word 0)
-    REYN_CUDA(cudaMemsetAsync(status.get(), 0, (prekeyed ? 2 : 3) * sizeof(uint32_t), s));
+    if (status.size() < 2)
+        status.resize(2);
+    // the status bits (a pre-keyed build keeps word 1, the keys' status, which
+    // the scan folds into word 0)
+    REYN_CUDA(cudaMemsetAsync(status.get(), 0, (prekeyed ? 1 : 2) * sizeof(uint32_t), s));
     n = np;
     keys.resize(np);
     slots.resize(np);
     sorted.resize(np);
-    split.resize(np);
+    if (split.size() != np || split_dirty || unresolved) {
+        split.resize(np);
+        split.zero(s);
+    }
+    split_dirty = true;
+    unresolved = false;
     reordered = false;
     reordered_state = nullptr;
     built_pos[0] = x;
@@ -434,15 +437,13 @@ void Grid::build(const float* x, const float* y, const float* z, uint32_t np,
     if (np) {
         REYN_KERNEL("k_scatter", s,
             k_scatter_stable<<<blocks_for(np, THREADS), THREADS, 0, s>>>(np, keys.get(),
-            prefix.get(), counts.get(), slots.get(), sorted.get(), split.get(),
-            status.get() + 1));
-        // split cells are rare: a small fixed grid walks their list
-        REYN_KERNEL("k_rank_split", s,
-            k_rank_split<<<std::min<unsigned>(blocks_for(np, THREADS), 2 * 148), THREADS, 0,
-            s>>>(status.get() + 1, split.get(), slots.get(), keys.get(), prefix.get(),
-            sorted.get()));
+            prefix.get(), counts.get(), slots.get(), split.get()));
+        unresolved = true;
+        if (!reorder_follows) // else reorder_state's gather does it
+            resolve(s);
     }
     counts_dirty = false;
+    split_dirty = false;
 }
 
 // each point's scene from the scene offsets (binary search)
@@ -515,23 +516,34 @@ void Grid::check_status(cudaStream_t s, const char* what)
 
 // ---- gather / pack ----------------------------------------------------------
 
-__global__ void k_gather(uint32_t n, const uint32_t* __restrict__ perm, GatherArgs a)
+// dst[k][s] = src[k][perm[s]]; with RESOLVE perm is a build's slots, whose
+// canonical order is settled on the way (sorted is written): one launch less
+// than ranking the split cells first, which took 20 us for a million shuffled
+// particles and 5 to 8 for any number in order
+template <bool RESOLVE>
+__global__ void __launch_bounds__(THREADS) k_gather(uint32_t n,
+    const uint32_t* __restrict__ perm, GatherArgs a, SplitCells c)
 {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n)
         return;
     const uint32_t p = perm[s];
+    uint32_t d = s;
+    if constexpr (RESOLVE) {
+        d = canonical_slot(c, s, p);
+        c.sorted[d] = p;
+    }
     float v[MAX_GATHER];
 #pragma unroll
     for (int k = 0; k < MAX_GATHER; ++k)
         if (k < a.count) {
             v[k] = __ldg(a.src[k] + p);
-            a.dst[k][s] = v[k];
+            a.dst[k][d] = v[k];
         }
     if (a.pm)
-        a.pm[s] = make_float4(v[FX], v[FY], v[FZ], v[FM]);
+        a.pm[d] = make_float4(v[FX], v[FY], v[FZ], v[FM]);
     if (a.vel)
-        a.vel[s] = make_float4(v[FVX], v[FVY], v[FVZ], 0.f);
+        a.vel[d] = make_float4(v[FVX], v[FVY], v[FVZ], 0.f);
 }
 
 void launch_gather(uint32_t n, const uint32_t* perm, const GatherArgs& a, cudaStream_t s)
@@ -539,7 +551,7 @@ void launch_gather(uint32_t n, const uint32_t* perm, const GatherArgs& a, cudaSt
     if (!n)
         return;
     REYN_KERNEL("k_gather", s,
-        k_gather<<<blocks_for(n, THREADS), THREADS, 0, s>>>(n, perm, a));
+        k_gather<false><<<blocks_for(n, THREADS), THREADS, 0, s>>>(n, perm, a, SplitCells {}));
 }
 
 __global__ void k_pack(uint32_t n, const float* __restrict__ x, const float* __restrict__ y,
@@ -591,7 +603,15 @@ void reorder_state(reyn_particles& st, Grid& g, float* const* extra, uint32_t n_
     }
     a.pm = st.pm.get();
     a.vel = st.vel.get();
-    launch_gather(n, g.sorted.get(), a, s);
+    if (g.unresolved && n) {
+        REYN_KERNEL("k_gather", s,
+            k_gather<true><<<blocks_for(n, THREADS), THREADS, 0, s>>>(n, g.slots.get(), a,
+            SplitCells { g.slots.get(), g.split.get(), g.keys.get(), g.prefix.get(),
+                g.sorted.get() }));
+        g.unresolved = false;
+    } else {
+        launch_gather(n, g.sorted.get(), a, s);
+    }
     for (uint32_t k = 0; k < n_extra && n; ++k)
         REYN_CUDA(cudaMemcpyAsync(extra[k], extra_tmp.get() + size_t(k) * n,
             size_t(n) * sizeof(float), cudaMemcpyDeviceToDevice, s));
@@ -980,9 +1000,10 @@ void boundary_build(reyn_boundary& b, const float* bx, const float* by, const fl
     b.points.add(b.pm, nb);
     for (DevArray<float>* a : { &b.x, &b.y, &b.z, &b.m })
         b.points.add(*a, nb);
-    for (DevArray<uint32_t>* a : { &b.grid.keys, &b.grid.slots, &b.grid.sorted, &b.grid.split })
+    for (DevArray<uint32_t>* a : { &b.grid.keys, &b.grid.slots, &b.grid.sorted })
         b.points.add(*a, nb);
-    b.points.add(b.grid.status, 3);
+    b.points.add(b.grid.split, nb);
+    b.points.add(b.grid.status, 2);
     b.points.allocate();
     REYN_CUDA(cudaMemsetAsync(box.get(), 0xff, box.size() * sizeof(unsigned), s));
     if (n_scenes) {
@@ -1030,7 +1051,7 @@ void boundary_build(reyn_boundary& b, const float* bx, const float* by, const fl
     b.cells.add(b.grid.scan_part, scan_parts(C));
     b.cells.add(b.near, C);
     b.cells.allocate();
-    b.grid.counts_dirty = true; // not yet zero
+    b.grid.counts_dirty = b.grid.split_dirty = true; // not yet zero
     b.grid.build(bx, by, bz, nb, s);
     b.grid.check_status(s, "boundary grid");
     GatherArgs a {};

@@ -1810,12 +1810,12 @@ void solver_step_t(reyn_solver& sv, reyn_particles& st, const Grid& grid,
     // batch) computes the keys and histogram of that grid's next build
     const bool prekeyed = tail.vmax && !gx && !ns && !shadow && grid.n == n
         && grid.reordered_state == &st && !grid.counts_dirty && !grid.prekey_pending
-        && grid.counts.size() == size_t(grid.total_keys()) && grid.status.size() >= 3;
+        && grid.counts.size() == size_t(grid.total_keys()) && grid.status.size() >= 2;
     if (prekeyed) {
         tail.kg = grid.view(grid.geom.r);
         tail.keys = grid.keys.get();
         tail.counts = grid.counts.get();
-        tail.kstatus = grid.status.get() + 2;
+        tail.kstatus = grid.status.get() + 1;
     }
     const unsigned bs = P.block_size ? P.block_size : NBR_THREADS;
     const unsigned nb = blocks_for(n, bs);

@@ -94,7 +94,7 @@ extern "C" int reyn_autotune(reyn_scheme scheme, const reyn_params* params,
                 snap.restore(*state, s);
                 auto one = [&] {
                     grid.build(state->cur[FX].get(), state->cur[FY].get(), state->cur[FZ].get(),
-                        state->n, s);
+                        state->n, s, nullptr, true);
                     reorder_state(*state, grid, nullptr, 0, s);
                     try {
                         solver_step(sv, *state, grid, bdy, dt, s);
@@ -158,7 +158,7 @@ extern "C" int reyn_autotune_reorder(reyn_scheme scheme, const reyn_params* para
             snap.restore(*state, s);
             auto one = [&](bool reorder) {
                 grid.build(state->cur[FX].get(), state->cur[FY].get(), state->cur[FZ].get(),
-                    state->n, s);
+                    state->n, s, nullptr, reorder);
                 if (reorder)
                     reorder_state(*state, grid, nullptr, 0, s);
                 try {
