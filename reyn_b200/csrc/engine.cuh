@@ -79,7 +79,7 @@ struct Grid {
     DevArray<uint32_t> keys;   // n
     DevArray<uint32_t> slots;  // n, counting-sort output
     DevArray<uint32_t> sorted; // n, canonical order (the permutation)
-    DevArray<uint8_t> split;   // n, marks slots of cells split across warps
+    DevArray<uint8_t> split;   // n, marks slots of cells split across runs of lanes
     DevArray<uint32_t> scan_part;
     DevArray<uint32_t> status; // StatusBits, pre-key StatusBits
     DevArray<float> extra_tmp; // reorder staging of caller arrays

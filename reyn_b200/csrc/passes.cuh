@@ -1019,7 +1019,9 @@ unsigned persistent_grid(Kern kern, unsigned bs, unsigned tiles)
 // (SESPH): vel.w receives 1 / rho instead of rho. shift: warp_shift(n).
 // Bound by instruction issue (the cell traversal). One scene: held to 40
 // registers (12 blocks of 128 per SM); 48 registers run slower (514 against
-// 502 us on the 4M dam break in MIXED_POS16), 32 as well (527).
+// 502 us on the 4M dam break in MIXED_POS16), 32 as well (527). A batch takes
+// the compiler's choice: held to 40 or 48 it runs slower (1057 and 1028
+// against 1015 us over 96 scenes).
 template <int KIND, int R, bool XYZ, int MIX = 0, bool BATCH = false, int MB = NBR_THREADS>
 __global__ void __launch_bounds__(MB, (BATCH ? 0 : 65536 / 40 / MB))
 k_density(uint32_t n, Fluid f, Bdy b,
