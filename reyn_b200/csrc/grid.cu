@@ -75,29 +75,6 @@ namespace reyn {
 
 // ---- kernels --------------------------------------------------------------
 
-// The run of neighbouring lanes with this lane's key: its first lane, its
-// length and the lane's place in it. Particles in order hold a cell's indices
-// in a row, so runs find what __match_any_sync would at a fraction of its cost
-// (4M particles: keys 52 -> 29 us, scatter 46 -> 28); equal keys further apart
-// form runs of their own.
-struct Run {
-    int leader;
-    uint32_t len, rank;
-};
-
-__device__ __forceinline__ Run key_run(uint32_t key)
-{
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const uint32_t before = __shfl_up_sync(FULL, key, 1);
-    const unsigned heads = __ballot_sync(FULL, lane == 0 || before != key);
-    const unsigned upto = heads & (0xffffffffu >> (31 - lane));
-    const unsigned after = heads & ~(0xffffffffu >> (31 - lane));
-    const int leader = 31 - __clz(upto);
-    const int end = after ? __ffs(after) - 1 : 32;
-    return Run { leader, uint32_t(end - leader), uint32_t(lane - leader) };
-}
-
 // cell key of every particle + histogram (uniformgrid.cu:20-34), one atomic a
 // run of equal keys
 __global__ void k_keys_count(uint32_t n, const float* __restrict__ x,
