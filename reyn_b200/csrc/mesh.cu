@@ -173,55 +173,69 @@ namespace {
             leaf_test<INSIDE>(m, 0, p, best);
             return best;
         }
-        uint32_t st_node[STACK];
-        float st_dist[STACK];
-        st_node[0] = 0;
-        st_dist[0] = box_dist(m.root.lo[0], m.root.lo[1], m.root.lo[2], m.root.hi[0],
-            m.root.hi[1], m.root.hi[2], p);
-        int sp = 1;
-        auto visit = [&](uint32_t link, float dist) {
-            if (!(dist <= best.d2))
-                return;
-            const uint32_t k = link >> 1;
-            if (!(link & 1u)) {
-                if (k <= m.n_internal) // leaves 0 .. n_internal
-                    leaf_test<INSIDE>(m, k, p, best);
-                else
-                    atomicOr(m.status, MESH_BAD_TREE);
-            } else if (k >= m.n_internal) {
+        uint2 st[STACK]; // node, distance bits
+        int sp = 0;
+        auto leaf = [&](uint32_t k) {
+            if (k <= m.n_internal) // leaves 0 .. n_internal
+                leaf_test<INSIDE>(m, k, p, best);
+            else
                 atomicOr(m.status, MESH_BAD_TREE);
-            } else if (sp < STACK) {
-                st_node[sp] = k;
-                st_dist[sp] = dist;
-                ++sp;
-            } else {
-                atomicOr(m.status, MESH_STACK_FULL); // not for STACK >= height + 2
-            }
         };
+        uint32_t cur = 0;
+        if (box_dist(m.root.lo[0], m.root.lo[1], m.root.lo[2], m.root.hi[0], m.root.hi[1],
+                m.root.hi[2], p)
+            > best.d2)
+            return best;
         // a tree expands each internal node at most once
-        uint32_t pops = 0;
-        do {
-            if (++pops > m.n_internal) {
+        for (uint32_t left = m.n_internal;; --left) {
+            if (left == 0) {
                 atomicOr(m.status, MESH_BAD_TREE);
                 break;
             }
-            --sp;
-            if (st_dist[sp] > best.d2)
-                continue;
-            const Node* nd = m.nodes + st_node[sp];
+            const Node* nd = m.nodes + cur;
             const float4 a = __ldg(&nd->a), b = __ldg(&nd->b), c = __ldg(&nd->c);
             const uint4 d = __ldg(&nd->d);
             const float dl = box_dist(a.x, a.y, a.z, a.w, b.x, b.y, p);
             const float dr = box_dist(b.z, b.w, c.x, c.y, c.z, c.w, p);
-            // the farther child first, so that the nearer one is popped next
-            if (dl < dr) {
-                visit(d.y, dr);
-                visit(d.x, dl);
-            } else {
-                visit(d.x, dl);
-                visit(d.y, dr);
+            // the farther child waits on the stack (or is tested, if a leaf);
+            // the nearer one is next without a round trip through it, whose
+            // store and load would sit in the walk's chain of dependent loads
+            const bool l = dl < dr;
+            const uint32_t far = l ? d.y : d.x, near = l ? d.x : d.y;
+            const float fd = l ? dr : dl, nd2 = l ? dl : dr;
+            if (fd <= best.d2) {
+                const uint32_t k = far >> 1;
+                if (!(far & 1u))
+                    leaf(k);
+                else if (k >= m.n_internal)
+                    atomicOr(m.status, MESH_BAD_TREE);
+                else if (sp < STACK)
+                    st[sp++] = make_uint2(k, __float_as_uint(fd));
+                else
+                    atomicOr(m.status, MESH_STACK_FULL); // not for STACK >= height + 2
             }
-        } while (sp > 0);
+            bool down = false;
+            if (nd2 <= best.d2) {
+                const uint32_t k = near >> 1;
+                if (!(near & 1u))
+                    leaf(k);
+                else if (k >= m.n_internal)
+                    atomicOr(m.status, MESH_BAD_TREE);
+                else {
+                    cur = k;
+                    down = true;
+                }
+            }
+            if (down)
+                continue;
+            uint2 e;
+            do {
+                if (sp == 0)
+                    return best;
+                e = st[--sp];
+            } while (__uint_as_float(e.y) > best.d2);
+            cur = e.x;
+        }
         return best;
     }
 
