@@ -57,7 +57,14 @@ __host__ __device__ __forceinline__ float sat01(float a)
 
 template <int KIND> struct Shape;
 
+// w01 is w for q already in [0, 1]: the same value without the clamp
 template <> struct Shape<K_C2> { // w = (1-q)_+^4 (4q+1)
+    __device__ static float w01(float q)
+    {
+        const float t = 1.f - q;
+        const float t2 = t * t;
+        return t2 * t2 * (4.f * q + 1.f);
+    }
     __host__ __device__ static float w(float q)
     {
         const float t = fmaxf(0.f, 1.f - q);
@@ -79,6 +86,12 @@ template <> struct Shape<K_C2> { // w = (1-q)_+^4 (4q+1)
 };
 
 template <> struct Shape<K_B3> { // w = (1-q)_+^3 - 4 (1/2-q)_+^3
+    __device__ static float w01(float q)
+    {
+        const float t = 1.f - q;
+        const float u = sat01(0.5f - q);
+        return t * t * t - 4.f * u * u * u;
+    }
     __host__ __device__ static float w(float q)
     {
         const float t = fmaxf(0.f, 1.f - q);
@@ -94,6 +107,14 @@ template <> struct Shape<K_B3> { // w = (1-q)_+^3 - 4 (1/2-q)_+^3
 };
 
 template <> struct Shape<K_W6> { // w = (1-q)_+^8 (32q^3 + 25q^2 + 8q + 1)
+    __device__ static float w01(float q)
+    {
+        const float t = 1.f - q;
+        const float t2 = t * t;
+        const float t4 = t2 * t2;
+        const float q2 = q * q;
+        return (t4 * t4) * (32.f * q2 * q + 25.f * q2 + 8.f * q + 1.f);
+    }
     __host__ __device__ static float w(float q)
     {
         const float t = fmaxf(0.f, 1.f - q);
@@ -120,6 +141,7 @@ template <> struct Shape<K_W6> { // w = (1-q)_+^8 (32q^3 + 25q^2 + 8q + 1)
 };
 
 template <> struct Shape<K_COS> { // w = 4 cos(pi q) + cos(2 pi q) + 3
+    __device__ static float w01(float q) { return w(q); }
     __host__ __device__ static float w(float q)
     {
         const float s = (float)M_PI * fminf(1.f, q);
@@ -160,7 +182,7 @@ template <int KIND>
 __device__ __forceinline__ float pair_w(const KernelConst& k, float l2)
 {
     // l2 = 0: NaN saturates to q = 0
-    return k.w_scale * Shape<KIND>::w(__saturatef(mul_ftz(l2, rsqrt_ftz(l2)) * k.h_inv));
+    return k.w_scale * Shape<KIND>::w01(__saturatef(mul_ftz(l2, rsqrt_ftz(l2)) * k.h_inv));
 }
 
 template <int KIND, class = void> struct HasDwOverQ {
@@ -201,7 +223,7 @@ __device__ __forceinline__ void pair_wg(
 {
     const float inv = inv_length(l2);
     const float q = l2 * inv * k.h_inv;
-    w = k.w_scale * Shape<KIND>::w(__saturatef(q));
+    w = k.w_scale * Shape<KIND>::w01(__saturatef(q));
     g = k.dw_scale * Shape<KIND>::dw(q) * inv;
 }
 
@@ -474,22 +496,37 @@ __device__ __forceinline__ void for_each_row_xyz(const GridView& g, int3 c, floa
     }
 }
 
+// a0 - b0 and a1 - b1 in one packed instruction (each half rounded once)
+__device__ __forceinline__ void sub2(float a0, float a1, float b0, float b1, float& d0, float& d1)
+{
+    asm("{\n\t.reg .b64 a, b, m, d;\n\t"
+        "mov.b64 a, {%2, %3};\n\t"
+        "mov.b64 b, {%4, %5};\n\t"
+        "mov.b64 m, {%6, %6};\n\t"
+        "fma.rn.f32x2 d, b, m, a;\n\t"
+        "mov.b64 {%0, %1}, d;\n\t}"
+        : "=f"(d0), "=f"(d1)
+        : "f"(a0), "f"(a1), "f"(b0), "f"(b1), "f"(-1.f));
+}
+
 // Fixed-radius neighbour traversal: f(j, pts[j], dx, dy, dz, l2) for every
 // candidate with l2 <= r^2 (self included, as the reference's accumulation
 // does), in the reference's row order. `pts` are packed (x, y, z, mass) in
 // grid order.
 // XYZ: the grid is in XYZ order (the caller knows; false serves both orders).
-// On the 4M dam break from rest the density pass over these loops takes 502 us
+// On the 4M dam break from rest the density pass over these loops takes 491 us
 // against 747 us over for_each_row with the compiler's own unrolling of the
-// candidate loop (by four, for rows of three to five candidates); one
-// candidate a round 508 us, two with a clamped second index 566 us, five
+// candidate loop (by four, for rows of three to five candidates). Measured
+// when the loops below took 502 us: one candidate a round 508 us, two with a clamped second index 566 us, five
 // rows' candidates as 64-bit pointer loops 599 us, one load ahead 704 us.
 template <int R, bool XYZ = false, class F>
 __device__ __forceinline__ void for_each_neighbour(const GridView& g, int3 c,
     float xi, float yi, float zi, const float4* __restrict__ pts, F&& f)
 {
     auto test = [&](uint32_t j, const float4& q) {
-        const float dx = xi - q.x, dy_ = yi - q.y, dz_ = zi - q.z;
+        float dx, dy_;
+        sub2(xi, yi, q.x, q.y, dx, dy_);
+        const float dz_ = zi - q.z;
         const float l2 = fmaf(dx, dx, fmaf(dy_, dy_, dz_ * dz_));
         if (l2 <= g.r2)
             f(j, q, dx, dy_, dz_, l2);

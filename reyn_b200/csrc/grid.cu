@@ -768,14 +768,14 @@ __global__ void __launch_bounds__(NBR_THREADS) k_neighbour_stats(uint32_t n, Gri
     uint32_t cnt = 0;
     float l2sum = 0.f, dens = 0.f;
     for_each_neighbour<R, XYZ>(g, c, me.x, me.y, me.z, pts,
-        [&](uint32_t j, const float4& q, float, float, float, float l2) {
-            cnt += (j == s) ? 0u : 1u;
+        [&](uint32_t, const float4& q, float, float, float, float l2) {
+            cnt += 1u;
             l2sum += l2;
             if (rho)
                 dens += q.w * pair_w<KIND>(kc, l2);
         });
     if (count)
-        count[p] = cnt;
+        count[p] = cnt ? cnt - 1u : 0u; // without the point itself
     if (len2)
         len2[p] = l2sum;
     if (rho)
