@@ -141,6 +141,7 @@ struct reyn_particles {
     uint32_t n = 0;
     float rho0 = 1.f;
     std::array<reyn::DevArray<float>, reyn::NFIELDS> cur, alt;
+    reyn::Slab spare;           // the memory of alt, pm and vel (reserve_spare)
     reyn::DevArray<float4> pm;  // (x, y, z, m) in grid order
     reyn::DevArray<float4> vel; // (vx, vy, vz, rho)
     bool packed_valid = false;
@@ -168,6 +169,7 @@ struct reyn_solver {
     reyn_scheme scheme;
     reyn_params prm;
     uint32_t n = 0;
+    reyn::Slab store; // the memory of the per-particle buffers (ensure_buffers)
     reyn::DevArray<float> rho, p, aii, sii, ax, ay, az;
     reyn::DevArray<float4> acc, vel2, bterm;
     reyn::DevArray<float> p_tmp;
@@ -228,6 +230,8 @@ void launch_gather(uint32_t n, const uint32_t* perm, const GatherArgs& a,
 void exclusive_scan(const uint32_t* in, int64_t C, DevArray<uint32_t>& part, uint32_t* out,
     cudaStream_t s, uint32_t* fold_status = nullptr);
 
+// the reorder's spare arrays and the packed copies, allocated together
+void reserve_spare(reyn_particles& st);
 // packs the particle arrays into pm/vel (after a direct SoA write)
 void pack_state(reyn_particles& st, cudaStream_t s);
 

@@ -217,10 +217,7 @@ extern "C" int reyn_step_graph_create(reyn_solver* sv, reyn_particles* st, reyn_
         // spare arrays, the solver's buffers and the batched and tail arrays
         const cudaStream_t s = gr->cap;
         g->build(st->cur[FX].get(), st->cur[FY].get(), st->cur[FZ].get(), st->n, s);
-        for (auto& a : st->alt)
-            a.resize(st->n);
-        st->pm.resize(st->n);
-        st->vel.resize(st->n);
+        reserve_spare(*st);
         g->extra_tmp.resize(st->n);
         ensure_buffers(*sv, st->n);
         const uint32_t ns = g->n_scenes;

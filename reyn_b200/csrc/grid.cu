@@ -573,15 +573,33 @@ void pack_state(reyn_particles& st, cudaStream_t s)
     st.packed_valid = true;
 }
 
+void reserve_spare(reyn_particles& st)
+{
+    const uint32_t n = st.n;
+    if (st.alt[0].size() == n && st.pm.size() == n && st.vel.size() == n)
+        return;
+    if (st.alt[0].size() || st.pm.size() || st.vel.size()) { // some are there already
+        for (auto& a : st.alt)
+            a.resize(n);
+        st.pm.resize(n);
+        st.vel.resize(n);
+        return;
+    }
+    Slab spare;
+    for (auto& a : st.alt)
+        spare.add(a, n);
+    spare.add(st.pm, n);
+    spare.add(st.vel, n);
+    spare.allocate();
+    st.spare = std::move(spare);
+}
+
 void reorder_state(reyn_particles& st, Grid& g, float* const* extra, uint32_t n_extra,
     cudaStream_t s)
 {
     require(n_extra + NFIELDS <= MAX_GATHER, "too many extra arrays to reorder (max 9)");
     const uint32_t n = st.n;
-    for (auto& a : st.alt)
-        a.resize(n);
-    st.pm.resize(n);
-    st.vel.resize(n);
+    reserve_spare(st);
     DevArray<float>& extra_tmp = g.extra_tmp;
     extra_tmp.resize(size_t(n) * std::max<uint32_t>(n_extra, 1));
     GatherArgs a {};
@@ -656,10 +674,7 @@ void reorder_by(reyn_particles& st, const uint32_t* sorted, cudaStream_t s)
             fail(REYN_ERR_INVALID, (host & 1u) ? "permutation index out of range"
                                                : "permutation repeats an index");
     }
-    for (auto& a : st.alt)
-        a.resize(n);
-    st.pm.resize(n);
-    st.vel.resize(n);
+    reserve_spare(st);
     GatherArgs a {};
     a.count = NFIELDS;
     for (int k = 0; k < NFIELDS; ++k) {
@@ -697,6 +712,7 @@ void resize_state(reyn_particles& st, uint32_t n, bool keep, cudaStream_t s)
     }
     st.pm = DevArray<float4>();
     st.vel = DevArray<float4>();
+    st.spare = Slab(); // no array lies in it any more
     st.n = n;
     st.packed_valid = false;
     st.epoch += 1;

@@ -59,36 +59,39 @@ double pcisph_template_delta(int kind, float h)
 
 void ensure_buffers(reyn_solver& sv, uint32_t n)
 {
-    sv.rho.resize(n);
-    sv.aii.resize(n);
-    sv.sii.resize(n);
-    sv.ax.resize(n);
-    sv.ay.resize(n);
-    sv.az.resize(n);
-    sv.vel2.resize(n);
-    sv.bterm.resize(n);
-    sv.nbr.resize(list_capacity(n));
-    sv.ncount.resize(n);
-    if (sv.prm.precision == REYN_PRECISION_MIXED) {
-        sv.acch.resize(n);
-        sv.velh.resize(n);
-        sv.velh2.resize(n);
-    } else if (sv.prm.precision == REYN_PRECISION_MIXED_POS16) {
-        sv.rec0.resize(n);
-        sv.rec1.resize(n);
-    }
-    if (sv.scheme == REYN_IISPH) {
-        sv.gq.resize(n);
-        if (sv.prm.precision != REYN_PRECISION_MIXED_POS16) {
-            sv.acc.resize(n);
-            sv.xq.resize(n);
+    if (sv.rho.size() != n) {
+        // every per-particle buffer in one allocation (a first step of a new
+        // solver otherwise waits for the allocator fifteen times)
+        Slab store;
+        for (DevArray<float>* a : { &sv.rho, &sv.aii, &sv.sii, &sv.ax, &sv.ay, &sv.az, &sv.p_tmp })
+            store.add(*a, n);
+        store.add(sv.vel2, n);
+        store.add(sv.bterm, n);
+        store.add(sv.nbr, list_capacity(n));
+        store.add(sv.ncount, n);
+        if (sv.prm.precision == REYN_PRECISION_MIXED) {
+            store.add(sv.acch, n);
+            store.add(sv.velh, n);
+            store.add(sv.velh2, n);
+        } else if (sv.prm.precision == REYN_PRECISION_MIXED_POS16) {
+            store.add(sv.rec0, n);
+            store.add(sv.rec1, n);
         }
+        if (sv.scheme == REYN_IISPH) {
+            store.add(sv.gq, n);
+            if (sv.prm.precision != REYN_PRECISION_MIXED_POS16) {
+                store.add(sv.acc, n);
+                store.add(sv.xq, n);
+            }
+        }
+        const bool fresh = sv.p.size() != n; // else a pressure was uploaded
+        if (fresh)
+            store.add(sv.p, n);
+        store.allocate();
+        sv.store = std::move(store);
+        if (fresh)
+            REYN_CUDA(cudaMemset(sv.p.get(), 0, size_t(n) * sizeof(float)));
     }
-    if (sv.p.size() != n) {
-        sv.p.resize(n);
-        REYN_CUDA(cudaMemset(sv.p.get(), 0, size_t(n) * sizeof(float)));
-    }
-    sv.p_tmp.resize(n);
     constexpr size_t SLOTS = 64;
     if (sv.sweep_stats.size() == 0) {
         sv.sweep_stats.resize(SLOTS * sizeof(SweepStats));
