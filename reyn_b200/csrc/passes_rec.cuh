@@ -36,7 +36,9 @@
 // 48 (214 us) and 40 (217 us, with spills): 209 us.
 template <int MB> constexpr int rec_min_blocks = 65536 / 56 / MB;
 // the batched forms (scene lookups, per-scene sums) are held to 64 registers,
-// 8 blocks of 128 per SM, against the 71 to 92 the compiler takes unbounded
+// 8 blocks of 128 per SM, against the 71 to 92 the compiler takes unbounded;
+// the non-pressure and final passes to 56 (306 -> 294 and 276 -> 260 us over 96
+// scenes; the diagonal pass loses there, 263 -> 284)
 
 // per-step constants of the record passes
 struct RecConst {
@@ -61,7 +63,7 @@ __device__ __forceinline__ float rec_m0(const Fluid& f)
 // 4 cells^2 / unit) where FP32 uses the IEEE one, since rho_j and v_j come
 // from FP16 already.
 template <int KIND, int R, bool BATCH, int MB>
-__global__ void __launch_bounds__(MB, (BATCH ? 65536 / 64 / MB : rec_min_blocks<MB>))
+__global__ void __launch_bounds__(MB, rec_min_blocks<MB>)
 k_np_rec(uint32_t n, Fluid f, RecConst rc,
     const float4* __restrict__ vel, const float4* __restrict__ bterm,
     const float* __restrict__ p_old, float nu10, float eps, float3 grav, float dt,
@@ -298,7 +300,7 @@ __device__ __forceinline__ void jacobi_rec(uint32_t i, REYN_JACOBI_REC_ARGS)
         emax = fmaxf(err, 0.f);
     }
     if constexpr (BATCH)
-        scene_accumulate(stats, sc, live, over, epos, 0.0, emax);
+        scene_accumulate_block(stats, sc, live, over, epos, emax);
     else
         block_accumulate(stats, over, epos, 0.0, emax);
 }
@@ -321,7 +323,7 @@ k_jacobi_rec_tiles(REYN_JACOBI_REC_ARGS, Tiles tl)
 // records; writes a (SoA) and the SoA state (bounds and the max |v|
 // reduction of a bounded step included)
 template <int KIND, int R, bool BATCH, int MB>
-__global__ void __launch_bounds__(MB, (BATCH ? 65536 / 64 / MB : rec_min_blocks<MB>))
+__global__ void __launch_bounds__(MB, rec_min_blocks<MB>)
 k_final_rec(uint32_t n, Fluid f, RecConst rc,
     const float4* __restrict__ gq, float r0i, const float4* __restrict__ vel, float dt,
     Soa3 acc, const uint4* __restrict__ rec_in, float* __restrict__ x,
