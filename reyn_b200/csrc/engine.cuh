@@ -227,6 +227,7 @@ void launch_gather(uint32_t n, const uint32_t* perm, const GatherArgs& a,
 
 // exclusive prefix sum of C counts into out[0..C] (out[C] = total); `part`
 // holds the per-tile partials
+size_t scan_parts(size_t C); // entries of `part` for C counts
 void exclusive_scan(const uint32_t* in, int64_t C, DevArray<uint32_t>& part, uint32_t* out,
     cudaStream_t s, uint32_t* fold_status = nullptr);
 

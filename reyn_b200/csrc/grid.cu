@@ -349,8 +349,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply(
         out[C] = total;
 }
 
-// the partial sums exclusive_scan needs for C counts
-static size_t scan_parts(size_t C) { return (C + SCAN_TILE - 1) / SCAN_TILE + 1; }
+size_t scan_parts(size_t C) { return (C + SCAN_TILE - 1) / SCAN_TILE + 1; }
 
 void exclusive_scan(const uint32_t* in, int64_t C, DevArray<uint32_t>& part,
     uint32_t* out, cudaStream_t s, uint32_t* fold_status)

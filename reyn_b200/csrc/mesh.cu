@@ -1004,25 +1004,21 @@ namespace {
     // scratch of a query batch in cell order (kept by the mesh, so that
     // the asynchronous queries never outlive it)
     struct QueryScratch {
-        DevArray<unsigned char> buf; // cells, pts
-        DevArray<uint32_t> part, counts, prefix;
-        uint32_t cap = 0;
-        uint32_t* cells = nullptr;
-        float4* pts = nullptr;
+        Slab store;
+        DevArray<uint32_t> cells, counts, prefix, part;
+        DevArray<float4> pts;
         void reserve(uint32_t n, int bits, cudaStream_t s)
         {
-            if (n > cap) {
-                Carve c;
-                const size_t oc = c.add<uint32_t>(n), op = c.add<float4>(n);
-                buf.resize(c.bytes);
-                cells = at<uint32_t>(buf, oc);
-                pts = at<float4>(buf, op);
-                cap = n;
-            }
             const size_t C = size_t(1) << bits;
-            if (counts.size() < C) {
-                counts.resize(C);
-                prefix.resize(C + 1);
+            if (n > pts.size() || C > counts.size()) {
+                Slab fresh; // one allocation
+                fresh.add(cells, n);
+                fresh.add(pts, n);
+                fresh.add(counts, C);
+                fresh.add(prefix, C + 1);
+                fresh.add(part, scan_parts(C));
+                fresh.allocate();
+                store = std::move(fresh);
             }
             REYN_CUDA(cudaMemsetAsync(counts.get(), 0, C * sizeof(uint32_t), s));
         }
@@ -1128,13 +1124,13 @@ void launch_query(const reyn_mesh& m, uint32_t n, const float4* src, const uint3
         }
         REYN_KERNEL("k_query_count", s,
             k_query_count<<<blocks_for(n, THREADS), THREADS, 0, s>>>(n, xin, yin, zin,
-            make_float3(lo[0], lo[1], lo[2]), make_float3(sc[0], sc[1], sc[2]), bits, q.cells,
+            make_float3(lo[0], lo[1], lo[2]), make_float3(sc[0], sc[1], sc[2]), bits, q.cells.get(),
             q.counts.get()));
         exclusive_scan(q.counts.get(), int64_t(1) << bits, q.part, q.prefix.get(), s);
         REYN_KERNEL("k_query_place", s,
-            k_query_place<<<blocks_for(n, THREADS), THREADS, 0, s>>>(n, q.cells, q.prefix.get(),
-            q.counts.get(), xin, yin, zin, q.pts));
-        src = q.pts;
+            k_query_place<<<blocks_for(n, THREADS), THREADS, 0, s>>>(n, q.cells.get(),
+            q.prefix.get(), q.counts.get(), xin, yin, zin, q.pts.get()));
+        src = q.pts.get();
     }
     const unsigned b = blocks_for(n, MESH_THREADS);
     if (m.stack() == 32)
