@@ -1944,9 +1944,11 @@ void solver_step_t(reyn_solver& sv, reyn_particles& st, const Grid& grid,
     f.acch = ACH;
     const Soa3 ACC { sv.ax.get(), sv.ay.get(), sv.az.get() };
     // FP32 and MIXED: the pressure passes' records (x, y, z, m p) in place of
-    // (x, y, z, m)
+    // (x, y, z, m); they take the memory of the packed velocities, which
+    // nothing reads after the non-pressure pass
+    float4* const XQ = st.vel.get();
     Fluid fq = f;
-    fq.pm = sv.xq.get();
+    fq.pm = XQ;
     auto body = [&](auto KC, auto RC, auto MC, auto BC) {
         constexpr int K = decltype(KC)::value;
         constexpr int R = decltype(RC)::value;
@@ -2173,7 +2175,7 @@ void solver_step_t(reyn_solver& sv, reyn_particles& st, const Grid& grid,
                 REYN_KERNEL("k_iisph_diag", s,
                     k_iisph_diag<K, R, MIX, B, MB><<<nb, bs, 0, s>>>(n, f, sv.vel2.get(),
                     VH2, sv.bterm.get(), sv.rho.get(), rho0, dt, P.omega, tiny, sv.aii.get(),
-                    sv.sii.get(), sv.p.get(), sv.gq.get(), sv.xq.get()));
+                    sv.sii.get(), sv.p.get(), sv.gq.get(), XQ));
                 pacc();
             }
             const float thr = P.eta * rho0;
@@ -2191,7 +2193,7 @@ void solver_step_t(reyn_solver& sv, reyn_particles& st, const Grid& grid,
                         launch_iisph_jacobi<K, R, MIX, B, MB>(nb, bs, q, tl, persist, n, f,
                         (const float4*)sv.acc.get(), (const float4*)sv.bterm.get(),
                         (const float*)sv.aii.get(), (const float*)sv.sii.get(), sv.p.get(),
-                        sv.xq.get(), dt, P.omega, tiny, thr, slot));
+                        XQ, dt, P.omega, tiny, thr, slot));
                     if (ns)
                         scene_converge_dev(q, P.convergence == REYN_CONV_AVERAGE ? 1 : 2);
                     decide(q, h, slot);
@@ -2206,7 +2208,7 @@ void solver_step_t(reyn_solver& sv, reyn_particles& st, const Grid& grid,
                     launch_iisph_jacobi<K, R, MIX, B, MB>(nb, bs, s, tl, persist, n, f,
                     (const float4*)sv.acc.get(), (const float4*)sv.bterm.get(),
                     (const float*)sv.aii.get(), (const float*)sv.sii.get(), sv.p.get(),
-                    sv.xq.get(), dt, P.omega, tiny, thr, slot));
+                    XQ, dt, P.omega, tiny, thr, slot));
                 iters += 1;
                 const bool last = max_it && iters >= max_it;
                 if (iters < P.min_iter && !last) {

@@ -79,10 +79,8 @@ void ensure_buffers(reyn_solver& sv, uint32_t n)
         }
         if (sv.scheme == REYN_IISPH) {
             store.add(sv.gq, n);
-            if (sv.prm.precision != REYN_PRECISION_MIXED_POS16) {
+            if (sv.prm.precision != REYN_PRECISION_MIXED_POS16)
                 store.add(sv.acc, n);
-                store.add(sv.xq, n);
-            }
         }
         const bool fresh = sv.p.size() != n; // else a pressure was uploaded
         if (fresh)
