@@ -174,6 +174,14 @@ __device__ __forceinline__ float mul_ftz(float a, float b)
     return r;
 }
 
+// 1 / a to 1 ulp for normal arguments, in one instruction
+__device__ __forceinline__ float rcp_ftz(float a)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+    return r;
+}
+
 // W and the gradient factor g (grad W = g * x_ij) for a neighbour pair with
 // squared distance 0 <= l2 <= r^2 (the traversal guarantees the range).
 // len = l2 * rsqrt(l2) replaces the reference's norm3df; the self pair

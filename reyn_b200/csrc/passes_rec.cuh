@@ -58,10 +58,11 @@ __device__ __forceinline__ float rec_m0(const Fluid& f)
 // record with m v* and m p_old for the diagonal pass. In record units the
 // viscosity term (10 nu m_j v_ij.x_ij g / (rho_j (|x_ij|^2 + eps))) x_ij
 // becomes (10 nu m_j v_ij.d g' / (rho_j (unit |d|^2 + eps / unit))) d. The
-// quotient is the fast division (2 ulp; its divisor stays far inside
-// [2^-126, 2^126] here: rho_j times a distance term between eps / unit and
-// 4 cells^2 / unit) where FP32 uses the IEEE one, since rho_j and v_j come
-// from FP16 already.
+// quotient is a product with the one-instruction reciprocal (1 ulp; its argument
+// stays far inside [2^-126, 2^126] here: rho_j times a distance term between
+// eps / unit and 4 cells^2 / unit) where FP32 uses the IEEE division, since
+// rho_j and v_j come from FP16 already; the pass is bound by issue (4M
+// particles 254 -> 246 us against the fast division's instructions).
 template <int KIND, int R, bool BATCH, int MB>
 __global__ void __launch_bounds__(MB, rec_min_blocks<MB>)
 k_np_rec(uint32_t n, Fluid f, RecConst rc,
@@ -88,7 +89,7 @@ k_np_rec(uint32_t n, Fluid f, RecConst rc,
             const float mg = rec_m16(rj) * g;
             const float vdx =
                 fmaf(vi.x - vxy.x, d.x, fmaf(vi.y - vxy.y, d.y, (vi.z - vzr.x) * d.z));
-            const float s = __fdividef(nu10 * mg * vdx, vzr.y * fmaf(rc.unit, l2, eps_u));
+            const float s = nu10 * mg * vdx * rcp_ftz(vzr.y * fmaf(rc.unit, l2, eps_u));
             ax += s * d.x;
             ay += s * d.y;
             az += s * d.z;
