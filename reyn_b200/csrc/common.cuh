@@ -32,11 +32,15 @@ void set_last_error(const std::string& msg);
     throw Error { code, msg };
 }
 
+// A failed call's error is reported here and taken off the runtime's record:
+// left there, the check after the next launch would report it again.
 inline void cuda_check(cudaError_t e, const char* what)
 {
-    if (e != cudaSuccess)
-        fail(e == cudaErrorMemoryAllocation ? REYN_ERR_ALLOC : REYN_ERR_CUDA,
-            std::string(what) + ": " + cudaGetErrorString(e));
+    if (e == cudaSuccess)
+        return;
+    (void)cudaGetLastError();
+    fail(e == cudaErrorMemoryAllocation ? REYN_ERR_ALLOC : REYN_ERR_CUDA,
+        std::string(what) + ": " + cudaGetErrorString(e));
 }
 
 #define REYN_CUDA(expr) ::reyn::cuda_check((expr), #expr)
