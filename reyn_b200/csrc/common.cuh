@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cstdint>
 #include <cstring>
 #include <exception>
@@ -198,6 +199,33 @@ private:
     size_t bytes_ = 0;
     std::vector<std::function<void(unsigned char*)>> parts_;
 };
+
+// The arrays a reorder writes to (its spare arrays and the packed copies), n
+// elements each: from one allocation, kept in `slab`, while none has memory yet,
+// else each by itself. An earlier call that ran out of memory may have left any
+// of them behind, so every one is asked for its size.
+template <size_t K>
+void reserve_together(size_t n, std::array<DevArray<float>, K>& alt, DevArray<float4>& pm,
+    DevArray<float4>& vel, Slab& slab)
+{
+    bool none = !pm.size() && !vel.size();
+    for (auto& a : alt)
+        none = none && !a.size();
+    if (!none || !n) {
+        for (auto& a : alt)
+            a.resize(n);
+        pm.resize(n);
+        vel.resize(n);
+        return;
+    }
+    Slab fresh;
+    for (auto& a : alt)
+        fresh.add(a, n);
+    fresh.add(pm, n);
+    fresh.add(vel, n);
+    fresh.allocate();
+    slab = std::move(fresh);
+}
 
 // Pinned host scratch for small device->host readbacks.
 template <class T> class PinnedArray {

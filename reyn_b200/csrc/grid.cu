@@ -574,23 +574,7 @@ void pack_state(reyn_particles& st, cudaStream_t s)
 
 void reserve_spare(reyn_particles& st)
 {
-    const uint32_t n = st.n;
-    if (st.alt[0].size() == n && st.pm.size() == n && st.vel.size() == n)
-        return;
-    if (st.alt[0].size() || st.pm.size() || st.vel.size()) { // some are there already
-        for (auto& a : st.alt)
-            a.resize(n);
-        st.pm.resize(n);
-        st.vel.resize(n);
-        return;
-    }
-    Slab spare;
-    for (auto& a : st.alt)
-        spare.add(a, n);
-    spare.add(st.pm, n);
-    spare.add(st.vel, n);
-    spare.allocate();
-    st.spare = std::move(spare);
+    reserve_together(st.n, st.alt, st.pm, st.vel, st.spare);
 }
 
 void reorder_state(reyn_particles& st, Grid& g, float* const* extra, uint32_t n_extra,

@@ -70,9 +70,45 @@ static void reported_once()
     g_allocs_left = -1;
 }
 
+// the arrays of a reorder, some of which an earlier step already holds: a call
+// that runs out of memory is refused, and so is the next one, until every array
+// has its memory
+static void reorder_arrays()
+{
+    for (int ok = 0; ok < 7; ++ok) {
+        std::array<DevArray<float>, 7> alt;
+        DevArray<float4> pm, vel;
+        Slab slab;
+        pm.resize(100);
+        vel.resize(100);
+        g_allocs_left = ok;
+        auto reserve = [&] { reserve_together(100, alt, pm, vel, slab); };
+        expect(throws(reserve), "out of memory is reported");
+        expect(throws(reserve), "and reported again while it lasts");
+        g_allocs_left = -1;
+        expect(!throws(reserve), "memory again");
+        for (auto& a : alt)
+            expect(a.get() != nullptr && a.size() == 100, "every array has its memory");
+    }
+    // fresh: one allocation for all, none kept of a failed one
+    std::array<DevArray<float>, 7> alt;
+    DevArray<float4> pm, vel;
+    Slab slab;
+    g_allocs_left = 0;
+    expect(throws([&] { reserve_together(100, alt, pm, vel, slab); }), "nothing fits");
+    g_allocs_left = 1;
+    expect(!throws([&] { reserve_together(100, alt, pm, vel, slab); }), "one allocation");
+    reserve_together(100, alt, pm, vel, slab);
+    for (auto& a : alt)
+        expect(a.get() != nullptr && a.size() == 100, "every array has its memory");
+    expect(pm.get() && vel.get(), "the packed copies too");
+    g_allocs_left = -1;
+}
+
 int main()
 {
     reported_once();
+    reorder_arrays();
     expect(g_live.empty(), "every allocation was freed");
     return failures;
 }
