@@ -2248,6 +2248,9 @@ void solver_step_t(reyn_solver& sv, reyn_particles& st, const Grid& grid,
                 VX, VY, VZ, tail));
         }
     };
+    // the passes overwrite the packed copies and then move the positions: a step
+    // that ends early must not leave them marked as the state's
+    st.packed_valid = false;
     dispatch(P.kernel, grid.geom.range, [&](auto KC, auto RC) {
         // batched scenes: the records of the mixed modes use each scene's own
         // grid origin (the cell size is shared), and neighbours never cross
@@ -2265,7 +2268,6 @@ void solver_step_t(reyn_solver& sv, reyn_particles& st, const Grid& grid,
         else
             body(KC, RC, std::integral_constant<int, 0> {}, std::false_type {});
     });
-    st.packed_valid = false; // positions moved: the packed copy is stale
     st.version += 1;
     if (prekeyed) {
         Grid& gm = const_cast<Grid&>(grid);
