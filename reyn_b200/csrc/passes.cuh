@@ -1140,10 +1140,10 @@ __device__ __forceinline__ float pressure_term_sesph(float rho_inv, float k_r0, 
 // _compute_accelerations (SESPH.cu:15-65) fused with integrate (solver.cu:
 // 15-32): writes the new SoA state and the accelerations. vel.w is 1 / rho,
 // formed once per particle by the density pass: one quotient a pair instead
-// of the four that rho needs (a step of 1M particles 546 -> 497 us), and that
-// one a product with the one-instruction reciprocal (the pass over 32k particles
-// 21 -> 17 us; the accelerations' error against 64 bits stays 4.5e-7 for B3,
-// 6.1e-7 for C2, 8.6e-7 for C6).
+// of the four that rho needs (a step of 1M particles 546 -> 497 us). That one
+// is an IEEE division: a product with the one-instruction reciprocal is faster
+// (the pass over 32k particles 17 us instead of 21), but its error bound is three
+// times as large, and SESPH has no mode that lets a caller choose it.
 template <int KIND, int R, bool BATCH = false, int MB = NBR_THREADS>
 __global__ void __launch_bounds__(MB) k_sesph(uint32_t n, Fluid f,
     const float4* __restrict__ vel, const float4* __restrict__ bterm, float k_r0, float rho0,
@@ -1162,7 +1162,7 @@ __global__ void __launch_bounds__(MB) k_sesph(uint32_t n, Fluid f,
         [&](uint32_t j, const float4& q, float dx, float dy, float dz, float l2) {
             const float4 vj = __ldg(vel + j);
             const float vdx = fmaf(vi.x - vj.x, dx, fmaf(vi.y - vj.y, dy, (vi.z - vj.z) * dz));
-            const float visc = nu10 * vj.w * vdx * rcp_ftz(l2 + eps);
+            const float visc = nu10 * vj.w * vdx / (l2 + eps);
             const float prs = pri + pressure_term_sesph(vj.w, k_r0, rho0);
             const float s = q.w * (visc - prs) * pair_g<KIND>(f.kc, l2);
             ax += s * dx;
