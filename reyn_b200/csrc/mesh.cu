@@ -293,51 +293,194 @@ namespace {
         return v;
     }
 
-    // Query points are put in the order of coarse Morton cells (of the mesh's
-    // box, clamped), so that the lanes of a warp traverse similar paths: a
-    // counting sort by the leading `bits` bits of each point's Morton code, in
-    // any order inside a cell, since every query's result is its own.
-    __global__ void k_query_count(uint32_t n, const float* __restrict__ x,
-        const float* __restrict__ y, const float* __restrict__ z, float3 lo, float3 scale, int bits,
-        uint32_t* __restrict__ cells, uint32_t* __restrict__ counts)
-    {
-        const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-        const bool valid = i < n;
-        uint32_t cell = 0xffffffffu;
-        if (valid) {
+    // Query points are put in the order of Morton cells (of the mesh's box,
+    // clamped), so that the lanes of a warp traverse similar paths: a counting
+    // sort, in any order inside a cell, since every query's result is its own.
+    // The cells are as fine as the batch is dense: the box in 16^3 coarse cells,
+    // each cut into 8^k by the points it holds. Points gathered in a corner of the
+    // box are ordered like points all over it; with one cell size for the whole
+    // box they are not (2.5M queries in 1/512 of its edges: 1313 us, against 437
+    // by these cells and 541 by a radix sort of ten bits an axis).
+    constexpr int COARSE_BITS = 12;
+    constexpr uint32_t COARSE_CELLS = 1u << COARSE_BITS;
+    constexpr int FINE_LEVELS = 9; // a coarse cell's edge in 512: 13 bits an axis in all
+    constexpr int QUERY_THREADS = 512;
+
+    // a point's place in the box, 13 bits an axis (rounded explicitly: three
+    // kernels have to agree on it)
+    struct QueryBox {
+        float3 lo, scale;
+        __device__ uint3 at(float x, float y, float z) const
+        {
             auto q = [](float v, float l, float sc) {
-                const float t = (v - l) * sc;
-                return uint32_t(fminf(fmaxf(t, 0.f), 1023.f)); // NaN -> 0
+                constexpr float LAST = (1 << (COARSE_BITS / 3 + FINE_LEVELS)) - 1;
+                const float u = __fmul_rn(__fsub_rn(v, l), sc);
+                return uint32_t(fminf(fmaxf(u, 0.f), LAST)); // NaN -> 0
             };
-            cell = ((spread10(q(x[i], lo.x, scale.x)) << 2)
-                       | (spread10(q(y[i], lo.y, scale.y)) << 1)
-                       | spread10(q(z[i], lo.z, scale.z)))
-                >> (30 - bits);
-            cells[i] = cell;
+            return make_uint3(q(x, lo.x, scale.x), q(y, lo.y, scale.y), q(z, lo.z, scale.z));
         }
-        const Run r = key_run(cell);
-        if (valid && r.rank == 0)
-            atomicAdd(counts + cell, r.len);
+    };
+
+    __device__ __forceinline__ uint32_t morton(uint3 p)
+    {
+        return (spread10(p.x) << 2) | (spread10(p.y) << 1) | spread10(p.z);
     }
 
-    // the point, with its index in w, to a place of its cell; the cells' counts
-    // return to zero
-    __global__ void k_query_place(uint32_t n, const uint32_t* __restrict__ cells,
-        const uint32_t* __restrict__ prefix, uint32_t* __restrict__ counts,
+    __device__ __forceinline__ uint32_t coarse_cell(uint3 p)
+    {
+        return morton(make_uint3(p.x >> FINE_LEVELS, p.y >> FINE_LEVELS, p.z >> FINE_LEVELS));
+    }
+
+    // the points of each coarse cell: a block counts in shared memory (gathered
+    // points would meet on a few global counters)
+    __global__ void __launch_bounds__(QUERY_THREADS) k_query_count(uint32_t n,
+        const float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ z,
+        QueryBox box, uint32_t* __restrict__ coarse)
+    {
+        __shared__ uint32_t h[COARSE_CELLS];
+        for (uint32_t c = threadIdx.x; c < COARSE_CELLS; c += QUERY_THREADS)
+            h[c] = 0u;
+        __syncthreads();
+        for (size_t i = size_t(blockIdx.x) * QUERY_THREADS + threadIdx.x; i < n;
+             i += size_t(gridDim.x) * QUERY_THREADS)
+            atomicAdd(h + coarse_cell(box.at(x[i], y[i], z[i])), 1u);
+        __syncthreads();
+        for (uint32_t c = threadIdx.x; c < COARSE_CELLS; c += QUERY_THREADS)
+            if (h[c])
+                atomicAdd(coarse + c, h[c]);
+    }
+
+    // The cells of a coarse cell with `pts` points: 8^k, the most that keep 8^k <=
+    // density * pts, so that at most density * n cells are used in all.
+    __device__ __forceinline__ uint32_t split_levels(uint32_t pts, uint32_t density)
+    {
+        return pts ? min(FINE_LEVELS, (31 - __clz(pts * density)) / 3) : 0u;
+    }
+
+    // the cell of a point: its coarse cell's first one, then the leading bits of
+    // its place in the coarse cell
+    __device__ __forceinline__ uint32_t fine_cell(uint3 p, uint32_t first, uint32_t levels)
+    {
+        constexpr uint32_t FINE = (1u << FINE_LEVELS) - 1u;
+        return first
+            + (morton(make_uint3(p.x & FINE, p.y & FINE, p.z & FINE))
+                >> (3 * (FINE_LEVELS - levels)));
+    }
+
+    // Each point's place among its cell's points, and the cells' counts. A block
+    // first finds the coarse cells' first cells (a scan of 4096 counts costs it less
+    // than a launch of its own) and passes them on in `split`. Its points meet in
+    // a table of cells in shared memory, which takes one range of each cell's
+    // places for all of them: with an atomic a point, points gathered in a few
+    // cells wait for those cells' counters (2.5M points in thirty cells: 430 us).
+    // A cell that finds its entry taken by another goes to the global counter.
+    constexpr int REFINE_ITEMS = 4;
+    constexpr int REFINE_TILE = QUERY_THREADS * REFINE_ITEMS;
+    constexpr int REFINE_TABLE_BITS = 11;
+
+    __global__ void __launch_bounds__(QUERY_THREADS) k_query_refine(uint32_t n,
+        const float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ z,
+        QueryBox box, uint32_t density, const uint32_t* __restrict__ coarse,
+        uint2* __restrict__ split, uint32_t* __restrict__ places, uint32_t* __restrict__ counts)
+    {
+        constexpr uint32_t TABLE = 1u << REFINE_TABLE_BITS, NONE = 0xffffffffu;
+        constexpr int PER = COARSE_CELLS / QUERY_THREADS, W = QUERY_THREADS / 32;
+        __shared__ uint32_t first[COARSE_CELLS];
+        __shared__ uint8_t levels[COARSE_CELLS];
+        __shared__ uint32_t key[TABLE], taken[TABLE];
+        __shared__ uint32_t warp_tot[W];
+        const uint32_t t = threadIdx.x;
+        for (uint32_t h = t; h < TABLE; h += QUERY_THREADS) {
+            key[h] = NONE;
+            taken[h] = 0u;
+        }
+        static_assert(PER == 8, "two 16-byte loads of counts a thread");
+        const uint4 m0 = __ldg(reinterpret_cast<const uint4*>(coarse) + 2 * t);
+        const uint4 m1 = __ldg(reinterpret_cast<const uint4*>(coarse) + 2 * t + 1);
+        const uint32_t pts[PER] = { m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w };
+        uint32_t mine = 0;
+#pragma unroll
+        for (int c = 0; c < PER; ++c)
+            mine += pts[c] ? 1u << (3 * split_levels(pts[c], density)) : 0u;
+        const int lane = t & 31, w = t >> 5;
+        uint32_t inc = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o)
+                inc += u;
+        }
+        if (lane == 31)
+            warp_tot[w] = inc;
+        __syncthreads();
+        uint32_t at = inc - mine;
+        for (int k = 0; k < w; ++k)
+            at += warp_tot[k];
+#pragma unroll
+        for (int c = 0; c < PER; ++c) {
+            const uint32_t l = split_levels(pts[c], density);
+            first[t * PER + c] = at;
+            levels[t * PER + c] = uint8_t(l);
+            if (blockIdx.x == 0)
+                split[t * PER + c] = make_uint2(at, l);
+            at += pts[c] ? 1u << (3 * l) : 0u;
+        }
+        __syncthreads();
+
+        uint32_t entry[REFINE_ITEMS], place[REFINE_ITEMS];
+        const size_t i0 = size_t(blockIdx.x) * REFINE_TILE + t;
+#pragma unroll
+        for (int k = 0; k < REFINE_ITEMS; ++k) {
+            const size_t i = i0 + size_t(k) * QUERY_THREADS;
+            const bool valid = i < n;
+            uint32_t cell = NONE;
+            if (valid) {
+                const uint3 p = box.at(x[i], y[i], z[i]);
+                const uint32_t c = coarse_cell(p);
+                cell = fine_cell(p, first[c], levels[c]);
+            }
+            const Run r = key_run(cell);
+            uint32_t h = NONE, from = 0;
+            if (valid && r.rank == 0) {
+                h = (cell * 2654435769u) >> (32 - REFINE_TABLE_BITS);
+                const uint32_t was = atomicCAS(key + h, NONE, cell);
+                if (was == NONE || was == cell) {
+                    from = atomicAdd(taken + h, r.len);
+                } else {
+                    h = NONE;
+                    from = atomicAdd(counts + cell, r.len);
+                }
+            }
+            entry[k] = __shfl_sync(0xffffffffu, h, r.leader);
+            place[k] = __shfl_sync(0xffffffffu, from, r.leader) + r.rank;
+        }
+        __syncthreads();
+        for (uint32_t h = t; h < TABLE; h += QUERY_THREADS)
+            if (taken[h])
+                taken[h] = atomicAdd(counts + key[h], taken[h]);
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < REFINE_ITEMS; ++k) {
+            const size_t i = i0 + size_t(k) * QUERY_THREADS;
+            if (i < n)
+                places[i] = place[k] + (entry[k] == NONE ? 0u : taken[entry[k]]);
+        }
+    }
+
+    // the point, with its index in w, to its place of its cell
+    __global__ void k_query_place(uint32_t n, const uint2* __restrict__ split,
+        const uint32_t* __restrict__ places, const uint32_t* __restrict__ prefix, QueryBox box,
         const float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ z,
         float4* __restrict__ pts)
     {
         const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-        const bool valid = i < n;
-        const uint32_t cell = valid ? cells[i] : 0xffffffffu;
-        const Run r = key_run(cell);
-        uint32_t top = 0;
-        if (valid && r.rank == 0)
-            top = atomicSub(counts + cell, r.len);
-        top = __shfl_sync(0xffffffffu, top, r.leader);
-        if (valid)
-            pts[prefix[cell] + top - r.len + r.rank] =
-                make_float4(x[i], y[i], z[i], __uint_as_float(i));
+        if (i >= n)
+            return;
+        const float px = x[i], py = y[i], pz = z[i];
+        const uint3 p = box.at(px, py, pz);
+        const uint2 s = __ldg(split + coarse_cell(p));
+        pts[prefix[fine_cell(p, s.x, s.y)] + places[i]] =
+            make_float4(px, py, pz, __uint_as_float(i));
     }
 
     // ---- face areas, volume and the sampling CDF -----------------------------
@@ -1001,38 +1144,38 @@ namespace {
         z[o] = p.z;
     }
 
+    // cells a query batch may use: eight a point, fewer where that would take
+    // more than 2^24, and at least one. Never less for more points.
+    inline uint32_t query_cells(uint32_t n)
+    {
+        constexpr uint32_t MOST = 1u << 24;
+        return n <= MOST / 8 ? 8 * n : std::max(n, MOST);
+    }
+
     // scratch of a query batch in cell order (kept by the mesh, so that
     // the asynchronous queries never outlive it)
     struct QueryScratch {
         Slab store;
-        DevArray<uint32_t> cells, counts, prefix, part;
+        DevArray<uint32_t> places, tally, prefix, part;
+        DevArray<uint2> split;
         DevArray<float4> pts;
-        void reserve(uint32_t n, int bits, cudaStream_t s)
+        void reserve(uint32_t n)
         {
-            const size_t C = size_t(1) << bits;
-            if (n > pts.size() || C > counts.size()) {
-                Slab fresh; // one allocation
-                fresh.add(cells, n);
-                fresh.add(pts, n);
-                fresh.add(counts, C);
-                fresh.add(prefix, C + 1);
-                fresh.add(part, scan_parts(C));
-                fresh.allocate();
-                store = std::move(fresh);
-            }
-            REYN_CUDA(cudaMemsetAsync(counts.get(), 0, C * sizeof(uint32_t), s));
+            if (n <= pts.size())
+                return;
+            *this = QueryScratch(); // the smaller one first
+            const size_t C = query_cells(n);
+            Slab fresh; // one allocation
+            fresh.add(places, n);
+            fresh.add(pts, n);
+            fresh.add(tally, COARSE_CELLS + C); // coarse cells' counts, then cells'
+            fresh.add(prefix, C + 1);
+            fresh.add(part, scan_parts(C));
+            fresh.add(split, COARSE_CELLS);
+            fresh.allocate();
+            store = std::move(fresh);
         }
     };
-
-    // Morton bits of the query cells: about one cell of the box a point, in
-    // whole levels (32k points 15 bits, 300k 21, from 2M on 24)
-    inline int query_bits(uint32_t n)
-    {
-        int bits = 15;
-        while (bits < 24 && (1u << bits) < n)
-            bits += 3;
-        return bits;
-    }
 
     // below this many points a query batch runs in the caller's order
     constexpr uint32_t QUERY_SORT_MIN = 1u << 15;
@@ -1111,25 +1254,31 @@ void launch_query(const reyn_mesh& m, uint32_t n, const float4* src, const uint3
         // queries in the order of Morton cells: the lanes of a warp then walk
         // nearly the same nodes, where random order makes each warp wait for its
         // costliest lane; results go back to the callers' slots. Over 300k points
-        // a counting sort of the cells takes 36 us, a radix sort of the whole
-        // codes (eighteen launches) 171.
+        // the order's kernels take 52 us, a radix sort of the whole codes
+        // (eighteen launches) 169; over 40k points 44 and 150.
         QueryScratch& q = m.query;
-        const int bits = query_bits(n);
-        q.reserve(n, bits, s);
+        q.reserve(n);
+        const uint32_t density = query_cells(n) / n, C = density * n;
         float lo[3], sc[3];
         for (int k = 0; k < 3; ++k) {
             lo[k] = float(m.lo[k]);
             const double ext = m.hi[k] - m.lo[k];
-            sc[k] = ext > 0.0 ? float(1024.0 / ext) : 0.f;
+            sc[k] = ext > 0.0 ? float(double(1 << (COARSE_BITS / 3 + FINE_LEVELS)) / ext) : 0.f;
         }
+        const QueryBox box { make_float3(lo[0], lo[1], lo[2]), make_float3(sc[0], sc[1], sc[2]) };
+        uint32_t* const coarse = q.tally.get();
+        uint32_t* const counts = coarse + COARSE_CELLS;
+        REYN_CUDA(cudaMemsetAsync(coarse, 0, (size_t(COARSE_CELLS) + C) * sizeof(uint32_t), s));
         REYN_KERNEL("k_query_count", s,
-            k_query_count<<<blocks_for(n, THREADS), THREADS, 0, s>>>(n, xin, yin, zin,
-            make_float3(lo[0], lo[1], lo[2]), make_float3(sc[0], sc[1], sc[2]), bits, q.cells.get(),
-            q.counts.get()));
-        exclusive_scan(q.counts.get(), int64_t(1) << bits, q.part, q.prefix.get(), s);
+            k_query_count<<<std::min(blocks_for(n, 4 * QUERY_THREADS), 1024u), QUERY_THREADS, 0,
+            s>>>(n, xin, yin, zin, box, coarse));
+        REYN_KERNEL("k_query_refine", s,
+            k_query_refine<<<blocks_for(n, REFINE_TILE), QUERY_THREADS, 0, s>>>(n, xin, yin, zin,
+            box, density, coarse, q.split.get(), q.places.get(), counts));
+        exclusive_scan(counts, int64_t(C), q.part, q.prefix.get(), s);
         REYN_KERNEL("k_query_place", s,
-            k_query_place<<<blocks_for(n, THREADS), THREADS, 0, s>>>(n, q.cells.get(),
-            q.prefix.get(), q.counts.get(), xin, yin, zin, q.pts.get()));
+            k_query_place<<<blocks_for(n, THREADS), THREADS, 0, s>>>(n, q.split.get(),
+            q.places.get(), q.prefix.get(), box, xin, yin, zin, q.pts.get()));
         src = q.pts.get();
     }
     const unsigned b = blocks_for(n, MESH_THREADS);
