@@ -896,18 +896,17 @@ __global__ void __launch_bounds__(THREADS) k_bounds(uint32_t n,
         atomicMin(box + 6 * sc + threadIdx.x, part[threadIdx.x]);
 }
 
-// one Akinci mass refinement (sample_boundary.cu:250-265), double-buffered:
-// m_i <- rho0 m_i / sum_j m_j W_B3(x_ij), support 2h; the last one also writes
-// the masses alone
+// one Akinci mass refinement (sample_boundary.cu:250-265): m_i <- rho0 m_i /
+// sum_j m_j W_B3(x_ij), support 2h, from the packed records into the masses
+// alone, which k_set_mass puts back into the records for the next one
 template <int R>
 __global__ void __launch_bounds__(NBR_THREADS) k_boundary_mass(uint32_t n, GridView g,
-    KernelConst kc, const float4* __restrict__ pts, float rho0, float4* __restrict__ out,
-    float* __restrict__ m_out)
+    KernelConst kc, const float4* __restrict__ pts, float rho0, float* __restrict__ m)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
         return;
-    g = at_scene(g, scene_of(g, i)); // batched boundaries: the sample's own scene
+    g = at_scene(g, scene_of(g, i)); // batched: the sample's own scene grid
     const float4 me = pts[i];
     int3 c = clamp_cell(g, cell_of(g, me.x, me.y, me.z), R);
     float sum = 0.f;
@@ -915,10 +914,14 @@ __global__ void __launch_bounds__(NBR_THREADS) k_boundary_mass(uint32_t n, GridV
         [&](uint32_t, const float4& q, float, float, float, float l2) {
             sum += q.w * pair_w<K_B3>(kc, l2);
         });
-    const float m = rho0 * me.w / sum;
-    out[i] = make_float4(me.x, me.y, me.z, m);
-    if (m_out)
-        m_out[i] = m;
+    m[i] = rho0 * me.w / sum;
+}
+
+__global__ void k_set_mass(uint32_t n, const float* __restrict__ m, float4* __restrict__ pts)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n)
+        pts[i].w = m[i];
 }
 
 // marks the (2R+1)^2 cells of every boundary sample's own x around it; the
@@ -984,12 +987,6 @@ void boundary_build(reyn_boundary& b, const float* bx, const float* by, const fl
     // once their number is known
     require(n_scenes <= 65535, "1 .. 65535 scenes");
     const uint32_t ns = std::max(1u, n_scenes);
-    DevArray<unsigned> box;
-    DevArray<uint32_t> sfirst;
-    DevArray<float4> other;
-    b.points.add(box, size_t(6) * ns);
-    b.points.add(sfirst, n_scenes ? n_scenes + 1 : 0);
-    b.points.add(other, bm ? 0 : nb);
     b.points.add(b.pm, nb);
     for (DevArray<float>* a : { &b.x, &b.y, &b.z, &b.m })
         b.points.add(*a, nb);
@@ -998,20 +995,29 @@ void boundary_build(reyn_boundary& b, const float* bx, const float* by, const fl
     b.points.add(b.grid.split, nb);
     b.points.add(b.grid.status, 2);
     b.points.allocate();
-    REYN_CUDA(cudaMemsetAsync(box.get(), 0xff, box.size() * sizeof(unsigned), s));
+    // the scenes' boxes and offsets are needed before the packed records: they
+    // take their memory, where it is enough
+    const size_t box_words = size_t(6) * ns, first_words = n_scenes ? n_scenes + 1 : 0;
+    DevArray<uint32_t> apart;
+    uint32_t* box = reinterpret_cast<uint32_t*>(b.pm.get());
+    if (box_words + first_words > size_t(4) * nb) {
+        apart.resize(box_words + first_words);
+        box = apart.get();
+    }
+    uint32_t* const sfirst = box + box_words;
+    REYN_CUDA(cudaMemsetAsync(box, 0xff, box_words * sizeof(uint32_t), s));
     if (n_scenes) {
         for (uint32_t k = 0; k < n_scenes; ++k)
             require(scene_first[k + 1] > scene_first[k],
                 "every scene of a batched boundary needs samples");
-        REYN_CUDA(cudaMemcpyAsync(sfirst.get(), scene_first, (n_scenes + 1) * sizeof(uint32_t),
+        REYN_CUDA(cudaMemcpyAsync(sfirst, scene_first, (n_scenes + 1) * sizeof(uint32_t),
             cudaMemcpyHostToDevice, s));
     }
     const dim3 bgrid(std::min(blocks_for(nb / ns + 1, THREADS * 4), 148u * 4u), ns);
     REYN_KERNEL("k_bounds", s,
-        k_bounds<<<bgrid, THREADS, 0, s>>>(nb, n_scenes ? sfirst.get() : nullptr, bx, by, bz,
-        box.get()));
-    std::vector<unsigned> hb(box.size());
-    REYN_CUDA(cudaMemcpyAsync(hb.data(), box.get(), hb.size() * sizeof(unsigned),
+        k_bounds<<<bgrid, THREADS, 0, s>>>(nb, n_scenes ? sfirst : nullptr, bx, by, bz, box));
+    std::vector<unsigned> hb(box_words);
+    REYN_CUDA(cudaMemcpyAsync(hb.data(), box, hb.size() * sizeof(unsigned),
         cudaMemcpyDeviceToHost, s));
     REYN_CUDA(cudaStreamSynchronize(s));
     std::vector<float> los(size_t(3) * ns), his(size_t(3) * ns);
@@ -1082,9 +1088,9 @@ void boundary_build(reyn_boundary& b, const float* bx, const float* by, const fl
         for (uint32_t it = 0; it < mass_iters; ++it) {
             REYN_KERNEL("k_boundary_mass", s,
                 k_boundary_mass<2><<<blocks_for(nb, NBR_THREADS), NBR_THREADS, 0, s>>>(
-                nb, v, kc, b.pm.get(), rho0, other.get(),
-                it + 1 == mass_iters ? b.m.get() : nullptr));
-            b.pm.swap(other);
+                nb, v, kc, b.pm.get(), rho0, b.m.get()));
+            REYN_KERNEL("k_set_mass", s,
+                k_set_mass<<<blocks_for(nb, THREADS), THREADS, 0, s>>>(nb, b.m.get(), b.pm.get()));
         }
         REYN_CUDA(cudaStreamSynchronize(s));
     }
