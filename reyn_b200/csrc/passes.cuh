@@ -1319,7 +1319,8 @@ __global__ void k_advect(uint32_t n, const float4* __restrict__ pm,
 
 // The pressure passes of FP32 and MIXED read the neighbours' positions and
 // pressures as one record xq = (x, y, z, m p), with the gradient moment
-// G_i = sum_j m_j grad W_ij + g_b (gq) of the diagonal pass:
+// G_i = sum_j m_j grad W_ij + g_b of the diagonal pass (gm, kept in the SoA
+// accelerations until the final pass writes those):
 //   sum_j m_j (p_i + p_j) grad W_ij + p_i g_b = p_i G_i + sum_j (m_j p_j) grad W_ij
 // They are bound by the L1's gathers (a warp's 16-byte gather takes 8 to 16
 // wavefronts, a 4-byte one of p_j another 2 to 8), so one gather a pair
@@ -1335,7 +1336,7 @@ __global__ void __launch_bounds__(MB) k_iisph_diag(uint32_t n, Fluid f,
     const float4* __restrict__ vel, const uint2* __restrict__ velh,
     const float4* __restrict__ bterm, const float* __restrict__ rho, float rho0, float dt,
     float omega, float tiny, float* __restrict__ aii, float* __restrict__ sii,
-    float* __restrict__ p, float4* __restrict__ gq, float4* __restrict__ xq)
+    float* __restrict__ p, Soa3 gm, float4* __restrict__ xq)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
@@ -1370,7 +1371,9 @@ __global__ void __launch_bounds__(MB) k_iisph_diag(uint32_t n, Fluid f,
     const float s = (rho0 - rho[i]) / dt - (vdiv + fmaf(vi.x, bt.x, fmaf(vi.y, bt.y, vi.z * bt.z)));
     aii[i] = a;
     sii[i] = s;
-    gq[i] = make_float4(gx, gy, gz, 0.f);
+    gm.x[i] = gx;
+    gm.y[i] = gy;
+    gm.z[i] = gz;
     const float pn = jacobi_update(omega, a, 0.f, s, tiny);
     p[i] = pn;
     xq[i] = make_float4(me.x, me.y, me.z, me.w * pn);
@@ -1387,7 +1390,7 @@ __global__ void __launch_bounds__(MB) k_iisph_diag_pacc(uint32_t n, Fluid f,
     const float4* __restrict__ vel, const uint2* __restrict__ velh,
     const float4* __restrict__ bterm, const float* __restrict__ rho, float rho0, float dt,
     float r0i, const float* __restrict__ p_old, float* __restrict__ aii,
-    float* __restrict__ sii, float* __restrict__ p_new, float4* __restrict__ gq,
+    float* __restrict__ sii, float* __restrict__ p_new, Soa3 gm,
     float4* __restrict__ acc, uint2* __restrict__ acch_out)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1425,7 +1428,9 @@ __global__ void __launch_bounds__(MB) k_iisph_diag_pacc(uint32_t n, Fluid f,
     gx += bt.x;
     gy += bt.y;
     gz += bt.z;
-    gq[i] = make_float4(gx, gy, gz, 0.f);
+    gm.x[i] = gx;
+    gm.y[i] = gy;
+    gm.z[i] = gz;
     const float4 ai = make_float4(-r0i * fmaf(pi, gx, 0.5f * sx), -r0i * fmaf(pi, gy, 0.5f * sy),
         -r0i * fmaf(pi, gz, 0.5f * sz), 0.f);
     acc[i] = ai;
@@ -1454,7 +1459,7 @@ __device__ __forceinline__ float3 pressure_sum(const Fluid& f, uint32_t i, const
 
 template <int KIND, int R, int MIX, bool BATCH>
 __device__ __forceinline__ void iisph_pacc(uint32_t i, uint32_t n, const Fluid& f,
-    const float* __restrict__ p, const float4* __restrict__ gq, float r0i,
+    const float* __restrict__ p, Soa3 gm, float r0i,
     float4* __restrict__ acc, uint2* __restrict__ acch_out, const uint32_t* __restrict__ gate)
 {
     // a captured step's loop body: the first sweep uses the accelerations of
@@ -1468,9 +1473,8 @@ __device__ __forceinline__ void iisph_pacc(uint32_t i, uint32_t n, const Fluid& 
     const float4 me = f.pm[i];
     const float3 s = pressure_sum<KIND, R, MIX, BATCH>(f, i, me);
     const float pi = p[i];
-    const float4 G = gq[i];
-    const float4 ai = make_float4(-r0i * fmaf(pi, G.x, s.x), -r0i * fmaf(pi, G.y, s.y),
-        -r0i * fmaf(pi, G.z, s.z), 0.f);
+    const float4 ai = make_float4(-r0i * fmaf(pi, gm.x[i], s.x), -r0i * fmaf(pi, gm.y[i], s.y),
+        -r0i * fmaf(pi, gm.z[i], s.z), 0.f);
     acc[i] = ai;
     if constexpr (MIX)
         acch_out[i] = pack_acc(ai.x, ai.y, ai.z);
@@ -1538,10 +1542,10 @@ __device__ __forceinline__ void iisph_jacobi(uint32_t i, uint32_t n, const Fluid
 
 template <int KIND, int R, int MIX = 0, bool BATCH = false, int MB = NBR_THREADS>
 __global__ void __launch_bounds__(MB) k_iisph_pacc(uint32_t n, Fluid f,
-    const float* __restrict__ p, const float4* __restrict__ gq, float r0i,
+    const float* __restrict__ p, Soa3 gm, float r0i,
     float4* __restrict__ acc, uint2* __restrict__ acch_out, const uint32_t* __restrict__ gate)
 {
-    iisph_pacc<KIND, R, MIX, BATCH>(blockIdx.x * blockDim.x + threadIdx.x, n, f, p, gq, r0i,
+    iisph_pacc<KIND, R, MIX, BATCH>(blockIdx.x * blockDim.x + threadIdx.x, n, f, p, gm, r0i,
         acc, acch_out, gate);
 }
 
@@ -1557,11 +1561,11 @@ __global__ void __launch_bounds__(MB) k_iisph_jacobi(uint32_t n, Fluid f,
 
 template <int KIND, int R, int MIX, int MB>
 __global__ void __launch_bounds__(MB) k_iisph_pacc_tiles(uint32_t n, Fluid f,
-    const float* __restrict__ p, const float4* __restrict__ gq, float r0i,
+    const float* __restrict__ p, Soa3 gm, float r0i,
     float4* __restrict__ acc, uint2* __restrict__ acch_out, const uint32_t* __restrict__ gate,
     Tiles tl)
 {
-    REYN_TILE_LOOP(tl, (iisph_pacc<KIND, R, MIX, true>(i, n, f, p, gq, r0i, acc, acch_out,
+    REYN_TILE_LOOP(tl, (iisph_pacc<KIND, R, MIX, true>(i, n, f, p, gm, r0i, acc, acch_out,
         gate)));
 }
 
@@ -1587,10 +1591,10 @@ constexpr bool occupancy_variant = MIX != 0 && KIND != K_COS;
 
 template <int KIND, int R, int MIX, int MB>
 __global__ void __launch_bounds__(MB, (65536 / 40) / MB) k_iisph_pacc_occ(uint32_t n, Fluid f,
-    const float* __restrict__ p, const float4* __restrict__ gq, float r0i,
+    const float* __restrict__ p, Soa3 gm, float r0i,
     float4* __restrict__ acc, uint2* __restrict__ acch_out, const uint32_t* __restrict__ gate)
 {
-    iisph_pacc<KIND, R, MIX, false>(blockIdx.x * blockDim.x + threadIdx.x, n, f, p, gq, r0i,
+    iisph_pacc<KIND, R, MIX, false>(blockIdx.x * blockDim.x + threadIdx.x, n, f, p, gm, r0i,
         acc, acch_out, gate);
 }
 
@@ -1678,8 +1682,7 @@ void launch_nonpressure(unsigned nb, unsigned bs, cudaStream_t q, A... a)
 // accelerations go straight to the solver's SoA arrays
 template <int KIND, int R, int MIX = 0, bool BATCH = false, int MB = NBR_THREADS>
 __global__ void __launch_bounds__(MB) k_iisph_final(uint32_t n, Fluid f,
-    const float* __restrict__ p, const float4* __restrict__ gq, float r0i,
-    const float4* __restrict__ vel, float dt, Soa3 acc,
+    const float* __restrict__ p, float r0i, const float4* __restrict__ vel, float dt, Soa3 acc,
     float* __restrict__ x, float* __restrict__ y, float* __restrict__ z,
     float* __restrict__ vx, float* __restrict__ vy, float* __restrict__ vz, Tail tail)
 {
@@ -1689,10 +1692,10 @@ __global__ void __launch_bounds__(MB) k_iisph_final(uint32_t n, Fluid f,
     const float4 me = f.pm[i];
     const float3 s = pressure_sum<KIND, R, MIX, BATCH>(f, i, me);
     const float pi = p[i];
-    const float4 G = gq[i];
-    const float ax = -r0i * fmaf(pi, G.x, s.x);
-    const float ay = -r0i * fmaf(pi, G.y, s.y);
-    const float az = -r0i * fmaf(pi, G.z, s.z);
+    // acc holds G here
+    const float ax = -r0i * fmaf(pi, acc.x[i], s.x);
+    const float ay = -r0i * fmaf(pi, acc.y[i], s.y);
+    const float az = -r0i * fmaf(pi, acc.z[i], s.z);
     acc.x[i] = ax;
     acc.y[i] = ay;
     acc.z[i] = az;
@@ -2166,19 +2169,19 @@ void solver_step_t(reyn_solver& sv, reyn_particles& st, const Grid& grid,
             auto pacc = [&] {
                 REYN_KERNEL("k_iisph_pacc", s,
                     launch_iisph_pacc<K, R, MIX, B, MB>(nb, bs, s, tl, persist, n, fq, sv.p.get(),
-                    sv.gq.get(), r0i, sv.acc.get(), ACH, (const uint32_t*)nullptr));
+                    ACC, r0i, sv.acc.get(), ACH, (const uint32_t*)nullptr));
             };
             if (P.warmstart) {
                 REYN_KERNEL("k_iisph_diag_pacc", s,
                     k_iisph_diag_pacc<K, R, MIX, B, MB><<<nb, bs, 0, s>>>(n, f, sv.vel2.get(),
                     VH2, sv.bterm.get(), sv.rho.get(), rho0, dt, r0i, sv.p.get(), sv.aii.get(),
-                    sv.sii.get(), sv.p_tmp.get(), sv.gq.get(), sv.acc.get(), ACH));
+                    sv.sii.get(), sv.p_tmp.get(), ACC, sv.acc.get(), ACH));
                 sv.p.swap(sv.p_tmp);
             } else {
                 REYN_KERNEL("k_iisph_diag", s,
                     k_iisph_diag<K, R, MIX, B, MB><<<nb, bs, 0, s>>>(n, f, sv.vel2.get(),
                     VH2, sv.bterm.get(), sv.rho.get(), rho0, dt, P.omega, tiny, sv.aii.get(),
-                    sv.sii.get(), sv.p.get(), sv.gq.get(), XQ));
+                    sv.sii.get(), sv.p.get(), ACC, XQ));
                 pacc();
             }
             const float thr = P.eta * rho0;
@@ -2190,7 +2193,7 @@ void solver_step_t(reyn_solver& sv, reyn_particles& st, const Grid& grid,
                     SweepStats* slot = ns ? scene_slot : slots;
                     REYN_KERNEL("k_iisph_pacc", q,
                         launch_iisph_pacc<K, R, MIX, B, MB>(nb, bs, q, tl, persist, n, fq, sv.p.get(),
-                        sv.gq.get(), r0i, sv.acc.get(), ACH, (const uint32_t*)gx->gate));
+                        ACC, r0i, sv.acc.get(), ACH, (const uint32_t*)gx->gate));
                     REYN_CUDA(cudaMemsetAsync(slot, 0, sizeof(SweepStats) * (ns ? ns : 1), q));
                     REYN_KERNEL("k_iisph_jacobi", q,
                         launch_iisph_jacobi<K, R, MIX, B, MB>(nb, bs, q, tl, persist, n, f,
@@ -2243,9 +2246,8 @@ void solver_step_t(reyn_solver& sv, reyn_particles& st, const Grid& grid,
                 pacc();
             }
             REYN_KERNEL("k_iisph_final", s,
-                k_iisph_final<K, R, MIX, B, MB><<<nb, bs, 0, s>>>(n, fq, sv.p.get(), sv.gq.get(),
-                r0i, sv.vel2.get(), dt, ACC, X, Y, Z,
-                VX, VY, VZ, tail));
+                k_iisph_final<K, R, MIX, B, MB><<<nb, bs, 0, s>>>(n, fq, sv.p.get(), r0i,
+                sv.vel2.get(), dt, ACC, X, Y, Z, VX, VY, VZ, tail));
         }
     };
     // the passes overwrite the packed copies and then move the positions: a step

@@ -76,12 +76,10 @@ void ensure_buffers(reyn_solver& sv, uint32_t n)
         } else if (sv.prm.precision == REYN_PRECISION_MIXED_POS16) {
             store.add(sv.rec0, n);
             store.add(sv.rec1, n);
-        }
-        if (sv.scheme == REYN_IISPH) {
             store.add(sv.gq, n);
-            if (sv.prm.precision != REYN_PRECISION_MIXED_POS16)
-                store.add(sv.acc, n);
         }
+        if (sv.scheme == REYN_IISPH && sv.prm.precision != REYN_PRECISION_MIXED_POS16)
+            store.add(sv.acc, n);
         const bool fresh = sv.p.size() != n; // else a pressure was uploaded
         if (fresh)
             store.add(sv.p, n);
