@@ -299,7 +299,7 @@ namespace {
     // The cells are as fine as the batch is dense: the box in 16^3 coarse cells,
     // each cut into 8^k by the points it holds. Points gathered in a corner of the
     // box are ordered like points all over it; with one cell size for the whole
-    // box they are not (2.5M queries in 1/512 of its edges: 1313 us, against 437
+    // box they are not (2.5M queries in 1/512 of its edges: 1313 us, against 421
     // by these cells and 541 by a radix sort of ten bits an axis).
     constexpr int COARSE_BITS = 12;
     constexpr uint32_t COARSE_CELLS = 1u << COARSE_BITS;
@@ -390,6 +390,14 @@ namespace {
         __shared__ uint32_t key[TABLE], taken[TABLE];
         __shared__ uint32_t warp_tot[W];
         const uint32_t t = threadIdx.x;
+        const size_t i0 = size_t(blockIdx.x) * REFINE_TILE + t;
+        uint3 p[REFINE_ITEMS]; // on their way while the coarse cells are scanned
+#pragma unroll
+        for (int k = 0; k < REFINE_ITEMS; ++k) {
+            const size_t i = i0 + size_t(k) * QUERY_THREADS;
+            if (i < n)
+                p[k] = box.at(x[i], y[i], z[i]);
+        }
         for (uint32_t h = t; h < TABLE; h += QUERY_THREADS) {
             key[h] = NONE;
             taken[h] = 0u;
@@ -427,43 +435,49 @@ namespace {
         }
         __syncthreads();
 
-        uint32_t entry[REFINE_ITEMS], place[REFINE_ITEMS];
-        const size_t i0 = size_t(blockIdx.x) * REFINE_TILE + t;
+        // the items in step, so that their counters' answers come together
+        uint32_t cell[REFINE_ITEMS], entry[REFINE_ITEMS], place[REFINE_ITEMS];
+        Run r[REFINE_ITEMS];
 #pragma unroll
         for (int k = 0; k < REFINE_ITEMS; ++k) {
-            const size_t i = i0 + size_t(k) * QUERY_THREADS;
-            const bool valid = i < n;
-            uint32_t cell = NONE;
-            if (valid) {
-                const uint3 p = box.at(x[i], y[i], z[i]);
-                const uint32_t c = coarse_cell(p);
-                cell = fine_cell(p, first[c], levels[c]);
+            cell[k] = entry[k] = NONE;
+            if (i0 + size_t(k) * QUERY_THREADS < n) {
+                const uint32_t c = coarse_cell(p[k]);
+                cell[k] = fine_cell(p[k], first[c], levels[c]);
             }
-            const Run r = key_run(cell);
-            uint32_t h = NONE, from = 0;
-            if (valid && r.rank == 0) {
-                h = (cell * 2654435769u) >> (32 - REFINE_TABLE_BITS);
-                const uint32_t was = atomicCAS(key + h, NONE, cell);
-                if (was == NONE || was == cell) {
-                    from = atomicAdd(taken + h, r.len);
-                } else {
-                    h = NONE;
-                    from = atomicAdd(counts + cell, r.len);
-                }
+            r[k] = key_run(cell[k]);
+            if (cell[k] != NONE && r[k].rank == 0) {
+                const uint32_t h = (cell[k] * 2654435769u) >> (32 - REFINE_TABLE_BITS);
+                const uint32_t was = atomicCAS(key + h, NONE, cell[k]);
+                if (was == NONE || was == cell[k])
+                    entry[k] = h;
             }
-            entry[k] = __shfl_sync(0xffffffffu, h, r.leader);
-            place[k] = __shfl_sync(0xffffffffu, from, r.leader) + r.rank;
+        }
+#pragma unroll
+        for (int k = 0; k < REFINE_ITEMS; ++k) {
+            place[k] = 0u;
+            if (cell[k] != NONE && r[k].rank == 0)
+                place[k] = atomicAdd(entry[k] != NONE ? taken + entry[k] : counts + cell[k],
+                    r[k].len);
         }
         __syncthreads();
-        for (uint32_t h = t; h < TABLE; h += QUERY_THREADS)
-            if (taken[h])
-                taken[h] = atomicAdd(counts + key[h], taken[h]);
+        uint32_t got[TABLE / QUERY_THREADS];
+#pragma unroll
+        for (uint32_t q = 0; q < TABLE / QUERY_THREADS; ++q) {
+            const uint32_t h = t + q * QUERY_THREADS;
+            got[q] = taken[h] ? atomicAdd(counts + key[h], taken[h]) : 0u;
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < TABLE / QUERY_THREADS; ++q)
+            taken[t + q * QUERY_THREADS] = got[q];
         __syncthreads();
 #pragma unroll
         for (int k = 0; k < REFINE_ITEMS; ++k) {
+            const uint32_t e = __shfl_sync(0xffffffffu, entry[k], r[k].leader);
+            const uint32_t at0 = __shfl_sync(0xffffffffu, place[k], r[k].leader);
             const size_t i = i0 + size_t(k) * QUERY_THREADS;
             if (i < n)
-                places[i] = place[k] + (entry[k] == NONE ? 0u : taken[entry[k]]);
+                places[i] = at0 + r[k].rank + (e == NONE ? 0u : taken[e]);
         }
     }
 
@@ -1144,12 +1158,14 @@ namespace {
         z[o] = p.z;
     }
 
-    // cells a query batch may use: eight a point, fewer where that would take
-    // more than 2^24, and at least one. Never less for more points.
+    // cells a query batch may use: four a point, fewer where that would take
+    // more than 2^24, and at least one. Never less for more points. (The walk over
+    // 300k points near a surface or over the box is as long with one cell a point
+    // as with eight; gathered batches lose 10 % at one, 1 % at four.)
     inline uint32_t query_cells(uint32_t n)
     {
         constexpr uint32_t MOST = 1u << 24;
-        return n <= MOST / 8 ? 8 * n : std::max(n, MOST);
+        return n <= MOST / 4 ? 4 * n : std::max(n, MOST);
     }
 
     // scratch of a query batch in cell order (kept by the mesh, so that
@@ -1254,8 +1270,8 @@ void launch_query(const reyn_mesh& m, uint32_t n, const float4* src, const uint3
         // queries in the order of Morton cells: the lanes of a warp then walk
         // nearly the same nodes, where random order makes each warp wait for its
         // costliest lane; results go back to the callers' slots. Over 300k points
-        // the order's kernels take 52 us, a radix sort of the whole codes
-        // (eighteen launches) 169; over 40k points 44 and 150.
+        // the order's kernels take 44 us, a radix sort of the whole codes
+        // (eighteen launches) 169; over 40k points 41 and 150.
         QueryScratch& q = m.query;
         q.reserve(n);
         const uint32_t density = query_cells(n) / n, C = density * n;

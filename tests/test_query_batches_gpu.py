@@ -42,9 +42,9 @@ def test_one_mesh_many_batches(cuda):
     mesh.close()
 
 
-@pytest.mark.parametrize("n", [(1 << 21) - 1, (1 << 21) + 12345, 5_000_001])
+@pytest.mark.parametrize("n", [(1 << 21) + 12345, (1 << 22) - 1, (1 << 22) + 12345, 5_000_001])
 def test_large_batches_equal_small_ones(cuda, n):
-    """Around and above the size where a point has eight cells: the same points
+    """Around and above the size from which a point has fewer cells: the same points
     in pieces that run in the caller's order."""
     import torch
 
