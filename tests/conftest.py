@@ -13,6 +13,16 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "slow: full-size workloads")
 
 
+def pytest_collection_modifyitems(items):
+    """The comparisons with the reference's own PLY writer need its build, which
+    comes from the reference's sources and is not part of this repository."""
+    if os.path.exists(os.path.join(ROOT, "oracle", "_ref", "libreyn_ref.so")):
+        return
+    for it in items:
+        if it.name.startswith("test_ply_matches_reference_save_to_ply"):
+            it.add_marker(pytest.mark.skip(reason="oracle/_ref/libreyn_ref.so is not built"))
+
+
 @pytest.fixture(scope="session")
 def cuda():
     import torch
