@@ -524,9 +524,10 @@ __device__ __forceinline__ void sub2(float a0, float a1, float b0, float b1, flo
 // XYZ: the grid is in XYZ order (the caller knows; false serves both orders).
 // On the 4M dam break from rest the density pass over these loops takes 491 us
 // against 747 us over for_each_row with the compiler's own unrolling of the
-// candidate loop (by four, for rows of three to five candidates). Measured
-// when the loops below took 502 us: one candidate a round 508 us, two with a clamped second index 566 us, five
-// rows' candidates as 64-bit pointer loops 599 us, one load ahead 704 us.
+// candidate loop (by four, for rows of three to five candidates). Other forms,
+// measured when these loops took 502 us: one candidate a round 508 us, two with a
+// clamped second index 566 us, five rows' candidates as 64-bit pointer loops 599
+// us, one load ahead 704 us.
 template <int R, bool XYZ = false, class F>
 __device__ __forceinline__ void for_each_neighbour(const GridView& g, int3 c,
     float xi, float yi, float zi, const float4* __restrict__ pts, F&& f)

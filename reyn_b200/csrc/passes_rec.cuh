@@ -33,12 +33,13 @@
 // resident blocks the one-scene record passes are compiled for: 56 registers
 // a thread (9 blocks of 128 per SM). Measured on the 4M dam break against the
 // compiler's own choice (71 registers, 237 us per Jacobi sweep) and caps of
-// 48 (214 us) and 40 (217 us, with spills): 209 us.
+// 48 (214 us) and 40 (217 us, with spills): 209 us then, 194 since 1 / sqrt
+// takes one instruction.
 template <int MB> constexpr int rec_min_blocks = 65536 / 56 / MB;
 // the batched forms (scene lookups, per-scene sums) are held to 64 registers,
 // 8 blocks of 128 per SM, against the 71 to 92 the compiler takes unbounded;
-// the non-pressure and final passes to 56 (306 -> 294 and 276 -> 260 us over 96
-// scenes; the diagonal pass loses there, 263 -> 284)
+// the non-pressure and final passes to 56 (306 -> 299 and 276 -> 264 us over 96
+// scenes, 296 and 260 now; the diagonal pass loses there, 263 -> 284)
 
 // per-step constants of the record passes
 struct RecConst {
